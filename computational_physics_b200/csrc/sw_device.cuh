@@ -144,6 +144,49 @@ __device__ __forceinline__ void uf_union(uint32_t *p, uint32_t a, uint32_t b)
     }
 }
 
+constexpr uint32_t kNoLink = 0xFFFFFFFFu;  // a union linked no root
+
+// Unites a and b and returns the root it linked below the other (each root is linked at most once:
+// afterwards it is no root), or kNoLink when the two were already one tree.  Both walks advance
+// together, two levels a step, and leave every other node pointing at its grandparent: plain stores,
+// since a node that has a parent never becomes a root again and its grandparent stays its ancestor.
+__device__ __forceinline__ uint32_t uf_union_link(uint32_t *p, uint32_t a, uint32_t b)
+{
+    volatile uint32_t *vp = p;
+    while (true) {
+        const uint32_t ya = vp[a], yb = vp[b], za = vp[ya], zb = vp[yb];
+        if (za == zb)
+            return kNoLink;
+        if (ya == a && yb == b) {
+            const uint32_t lo = min(a, b), hi = max(a, b), old = atomicMin(p + hi, lo);
+            if (old == hi)
+                return hi;
+            a = lo;
+            b = old;
+            continue;
+        }
+        if (za != ya)
+            vp[a] = za;
+        if (zb != yb)
+            vp[b] = zb;
+        a = za;
+        b = zb;
+    }
+}
+
+// Points b straight at its root.  Every step is stored, so that when many nodes of a tree do this at
+// once each jumps over what the others have shortened: a chain of n links takes about log2 n steps.
+__device__ __forceinline__ void uf_flatten(uint32_t *p, const uint32_t b)
+{
+    volatile uint32_t *vp = p;
+    uint32_t y = vp[b], z = vp[y];
+    while (z != y) {
+        vp[b] = z;
+        y = z;
+        z = vp[y];
+    }
+}
+
 // ---- the same on the global label array, which other CTAs change concurrently.  Finds halve
 // the path as they go (x's parent becomes its grandparent); the update is an atomicMin, which
 // only ever moves a pointer to an ancestor, so it is safe against concurrent unions and keeps
@@ -182,8 +225,6 @@ __device__ __forceinline__ uint32_t guf_find(uint32_t *p, uint32_t x, const uint
     }
     return x;
 }
-
-constexpr uint32_t kNoLink = 0xFFFFFFFFu;  // guf_union_pair linked no root
 
 // The same union with the two root walks advancing together, one level per step, so the loads
 // of both chains are in flight at once.  Each step also points the node it leaves at its

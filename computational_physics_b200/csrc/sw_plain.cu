@@ -5,14 +5,11 @@
 // ising/src/swendsen_wang.cpp:94-112):
 //
 //   k_assign  [AssignLabels + the in-block part of MergeLabels]  one CTA per block of
-//             TBX x TBY tiles.  Each tile's lcg32 stream lives in the registers of one
-//             W-lane warp segment; the accept bits of every update are warp ballots.
-//             Spins of the block plus a one-site halo are staged in shared memory, bond
-//             words are formed bit-parallel, and a scanline pass with a lock-free union-find
-//             toward the minimum index labels the block in shared memory.  Writes each
+//             TBX x TBY tiles, one warp per 32-column strip (sw_strip.cuh): lcg32 draws, bond
+//             words and a scan with a lock-free union-find toward the minimum index.  Writes each
 //             site's label (block roots: their global index; other sites: the block-local
 //             index of their root) and the bond bits of the block's right and bottom edge.
-//             A recorded sweep (kDebug) labels tile by tile first, as the reference's
+//             A recorded sweep labels tile by tile instead (k_assign_tiles), as the reference's
 //             AssignLabels does, to dump that stage.
 //   k_merge   [MergeLabels across blocks]  atomicMin union on the global label array for
 //             the edge bonds recorded by k_assign; each union records the root it linked.
@@ -20,7 +17,7 @@
 //             cluster's minimum site index), which becomes its label.
 //   k_flip    [ResolveLabels + FlipClusters]  every site reads its block root's label;
 //             spin ^= root & 1.  (Without k_resolve, three kernels, k_flip walks the merged
-//             roots' chains itself: small lattices of blocks under 128 x 32 sites, see kResolveMinBlocks,
+//             roots' chains itself: lattices under kResolveMinSites sites,
 //             and the static-scratch entry point, which has no room for the linked roots.)
 //
 // k_measure (every measure_every-th sweep) reduces energy and magnetisation on the device
@@ -47,6 +44,7 @@
 
 #include "../../include/swb200.h"
 #include "sw_core.cuh"
+#include "sw_strip.cuh"
 
 namespace swb {
 
@@ -67,47 +65,64 @@ int fail(int code, const char *fmt, ...)
     return code;
 }
 
-constexpr uint32_t kAssignThreads = 512;  // at most this many lcg lanes per block
+constexpr uint32_t kTilesThreads = 512;  // CTA of the recorded sweep's assign
 
-// TXc, TYc make the tile shape a compile-time constant for the common shapes (0 = runtime).
-// `dump` is all null in a plain sweep; a recorded sweep runs the same instance with dumps on
-// (the tile-local stage only through the runtime-shape instance, which labels tile by tile).
-// kMeasure: the instance that also measures the spins it starts from (`meas`), used by the
-// sweep after a measured one; a separate instance so the others carry none of its registers.
-template <int W, int TXc, int TYc, bool kMeasure, bool kFixedOnly = false>
-__global__ void __launch_bounds__(kAssignThreads, 4) k_assign(const Geo g, const uint8_t *__restrict__ spins,
-                                                 uint32_t *__restrict__ labels, uint32_t *__restrict__ rng_state,
-                                                 uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter,
-                                                 const uint32_t thr, uint32_t *__restrict__ edge, const AssignDump dump,
-                                                 const MeasureArgs meas)
+// Bands of an assign block: one where the lattice's blocks fill the GPU with a warp per strip, else
+// a band per tile row (up to kBandsMax).
+constexpr uint32_t kFullBlocks = 592;
+inline uint32_t assign_bands(const Geo &g) { return g.nbx * g.nby >= kFullBlocks ? 1 : std::min(g.TBY, kBandsMax); }
+
+// The assign phase of a plain sweep (assign_strips): one warp per 32-column strip.  TXc, TYc: the tile
+// shape (TYc 0: any height).  `dump` is all null in a plain sweep; swb_sweep_dumped runs the same
+// instance with dumps on.  kMeasure: the instance that also measures the spins it starts from
+// (`meas`), used by the sweep after a measured one; a separate instance so the others carry none
+// of its registers.
+template <int W, int TXc, int TYc, bool kMeasure>
+__global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) k_assign(const Geo g, const uint8_t *spins,
+                                                              uint32_t *labels,
+                                                              uint32_t *__restrict__ rng_state,
+                                                              uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter,
+                                                              const uint32_t thr, uint32_t *edge,
+                                                              const AssignDump dump, const MeasureArgs meas, const uint32_t bands)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    assign_block<W, TXc, TYc, kFixedOnly, true, true, kFixedOnly>(g, blockIdx.x, blockIdx.y, spins, labels, rng_state,
-                                                             rng_sel, rng_iter, thr, edge, dump,
-                                                             kMeasure ? meas : MeasureArgs{}, smem);
+    assign_strips<W, TXc, TYc, kMeasure, true, true>(g, blockIdx.x, blockIdx.y, bands, spins, labels, rng_state, rng_sel,
+                                               rng_iter, thr, edge, dump, meas, smem);
 }
 
-__global__ void __launch_bounds__(256) k_merge(const Geo g, const uint32_t *__restrict__ edge, uint32_t *labels,
-                                               unsigned int *fault, uint32_t *__restrict__ linked)
+// The assign phase of swb_sweep_recorded, labelling tile by tile.
+template <int W>
+__global__ void __launch_bounds__(kTilesThreads) k_assign_tiles(const Geo g, const uint8_t *__restrict__ spins,
+                                                               uint32_t *__restrict__ labels,
+                                                               uint32_t *__restrict__ rng_state,
+                                                               uint8_t *__restrict__ rng_sel,
+                                                               uint32_t *__restrict__ rng_iter, const uint32_t thr,
+                                                               uint32_t *__restrict__ edge, const AssignDump dump)
 {
+    extern __shared__ __align__(16) unsigned char smem[];
+    assign_block_tiles<W>(g, blockIdx.x, blockIdx.y, spins, labels, rng_state, rng_sel, rng_iter, thr, edge, dump, smem);
+}
+
+__global__ void __launch_bounds__(256) k_merge(const Geo g, const uint32_t *edge, uint32_t *labels, unsigned int *fault,
+                                               uint32_t *linked)
+{
+    after_previous();
     merge_block(g, blockIdx.x, blockIdx.y, threadIdx.x, edge, labels, fault, linked);
 }
 
 // The linked roots of one block's merge slots (resolve_block), one thread per slot.
-__global__ void __launch_bounds__(256) k_resolve(const Geo g, const uint32_t *__restrict__ linked, uint32_t *labels,
+__global__ void __launch_bounds__(256) k_resolve(const Geo g, const uint32_t *linked, uint32_t *labels,
                                                  unsigned int *fault)
 {
+    after_previous();
     resolve_block(g, blockIdx.x, blockIdx.y, threadIdx.x, linked, labels, fault);
 }
 
 // Resolve + flip, one CTA per block (flip_block).
-// Lattices of full 128 x 32 blocks, or of at least kResolveMinBlocks blocks, resolve the
-// linked roots in k_resolve; others let k_flip chase them (one launch fewer).  Measured per
-// sweep on B200, chasing / resolving: 1024^2 tile 8 x 8 (512 blocks of 128 x 16, twice the
-// edge sites per site) 0.0367 / 0.0380 ms; 1024^2 tile 16 x 8 (256 blocks of 128 x 32)
-// 0.0356 / 0.0343 ms; 2048^2 0.0632 / 0.0598 ms; 4096^2 0.1733 / 0.1668 ms.
-constexpr uint32_t kResolveMinBlocks = 4096;
-constexpr uint32_t kResolveBlockSites = 128 * 32;
+// Lattices of at least kResolveMinSites sites resolve the linked roots in k_resolve; smaller ones
+// let k_flip chase them (one launch fewer).  Measured per sweep on B200, chasing / resolving:
+// 1024^2 34.5 / 34.7 us, 1500^2 (T = 2.0) 49.1 / 51.3, 2048^2 51.5 / 47.6, 4096^2 126.7 / 117.6.
+constexpr size_t kResolveMinSites = 2048u * 2048u;
 constexpr uint32_t kFlipThreads = 256;  // 6 CTAs per SM (40 registers), four quads of a 128 x 32 block per thread
 
 template <bool kWriteLabels, bool kResolved>
@@ -115,13 +130,15 @@ __global__ void __launch_bounds__(kFlipThreads, 6) k_flip(const Geo g, uint8_t *
                                                        unsigned int *fault)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    after_previous();
     flip_block<kWriteLabels, 4, kResolved>(g, blockIdx.x, blockIdx.y, spins, labels, fault, smem);
 }
 
-__global__ void __launch_bounds__(256) k_measure(const uint32_t L0, const uint32_t L1, const uint8_t *__restrict__ spins,
+__global__ void __launch_bounds__(256) k_measure(const uint32_t L0, const uint32_t L1, const uint8_t *spins,
                                                  Obs *obs, long long *series, const unsigned long long cap,
                                                  const int accumulate)
 {
+    after_previous();
     // work items: 64-site pieces of rows (row_em takes them 16 sites at a time); a thread's
     // partial sums stay far inside int range (at most 3 per site it visits)
     const size_t n = (size_t)L0 * L1;
@@ -193,7 +210,7 @@ struct swb_lattice {
     int device = 0;
     cudaStream_t stream = nullptr;
     Geo g{};
-    uint32_t W = 16, seed_base = 1, n_tiles = 0, n_blocks = 0, smem_assign = 0;
+    uint32_t W = 16, seed_base = 1, n_tiles = 0, n_blocks = 0, smem_assign = 0, bands = 1;
     size_t n = 0;
     uint8_t *spins = nullptr;
     uint32_t *labels = nullptr;
@@ -223,56 +240,42 @@ int set_device(const swb_lattice *h)
     return SWB_OK;
 }
 
+bool early_launch(const swb_lattice *h) { return h->g.nbx * h->g.nby < kEarlyBlocks; }
+
 template <int W, int TXc, int TYc>
 int launch_assign_k(swb_lattice *h, float p_add, const AssignDump &dump, const MeasureArgs &meas)
 {
     const Geo &g = h->g;
-    // Whole warps: the draws use full-warp shuffles and ballots; surplus lanes have no tile.
-    const dim3 grid(g.nbx, g.nby), block((g.TBX * g.TBY * W + 31) / 32 * 32);
-    if constexpr (W == 16 && TXc == 16 && TYc == 8) {
-        // every block a full 128 x 32 block of 512 threads: the fixed-only instance
-        if (g.BX == 128 && g.BY == 32 && g.L0 % 128 == 0 && g.L1 % 32 == 0 && block.x == 512) {
-            if (meas.obs)
-                k_assign<W, TXc, TYc, true, true><<<grid, block, h->smem_assign, h->stream>>>(
-                    g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add), h->edge,
-                    dump, meas);
-            else
-                k_assign<W, TXc, TYc, false, true><<<grid, block, h->smem_assign, h->stream>>>(
-                    g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add), h->edge,
-                    dump, meas);
-            SWB_LAUNCHED();
-            return SWB_OK;
-        }
-    }
-    if (meas.obs)
-        k_assign<W, TXc, TYc, true><<<grid, block, h->smem_assign, h->stream>>>(
-            g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add), h->edge, dump, meas);
-    else
-        k_assign<W, TXc, TYc, false><<<grid, block, h->smem_assign, h->stream>>>(
-            g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add), h->edge, dump, meas);
-    SWB_LAUNCHED();
-    return SWB_OK;
+    const dim3 grid(g.nbx, g.nby), block((g.BX + 31) / 32 * 32 * h->bands);
+    const uint32_t thr = accept_threshold(p_add);
+    auto k = meas.obs ? k_assign<W, TXc, TYc, true> : k_assign<W, TXc, TYc, false>;
+    return launch_next(early_launch(h), k, grid, block, h->smem_assign, h->stream, g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, thr,
+                       h->edge, dump, meas, h->bands);
 }
 
 // The instance a plain sweep of this handle runs (compile-time tile shape for the common
-// shapes), with `dump` passed through; a dump of the tile-local stage takes the runtime-shape
-// instance instead, whose tile-by-tile form computes that stage.
+// shapes), with `dump` passed through; a dump of the tile-local stage takes the kernel that labels
+// tile by tile instead.
 template <int W>
 int launch_assign_w(swb_lattice *h, float p_add, const AssignDump &dump, const MeasureArgs &meas)
 {
-    if (dump.tile_labels)
-        return launch_assign_k<W, 0, 0>(h, p_add, dump, meas);
+    const uint32_t tx = h->g.TX, ty = h->g.TY;
+    if (dump.tile_labels) {
+        // whole warps: the draws use full-warp shuffles and ballots; surplus lanes have no tile
+        const Geo &g = h->g;
+        k_assign_tiles<W><<<dim3(g.nbx, g.nby), std::min(kTilesThreads, (g.TBX * g.TBY * W + 31) / 32 * 32), assign_smem(g, W).total, h->stream>>>(
+            g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add), h->edge, dump);
+        SWB_LAUNCHED();
+        return SWB_OK;
+    }
     if constexpr (W == 16) {
-        const uint32_t tx = h->g.TX, ty = h->g.TY;
         if (tx == 16 && ty == 8) return launch_assign_k<W, 16, 8>(h, p_add, dump, meas);
         if (tx == 8 && ty == 8) return launch_assign_k<W, 8, 8>(h, p_add, dump, meas);
-        if (tx == 32 && ty == 4) return launch_assign_k<W, 32, 4>(h, p_add, dump, meas);
-        if (tx == 16 && ty == 16) return launch_assign_k<W, 16, 16>(h, p_add, dump, meas);
-        if (tx == 8 && ty == 16) return launch_assign_k<W, 8, 16>(h, p_add, dump, meas);
-        if (tx == 32 && ty == 8) return launch_assign_k<W, 32, 8>(h, p_add, dump, meas);
         if (tx == 16 && ty == 4) return launch_assign_k<W, 16, 4>(h, p_add, dump, meas);
     }
-    return launch_assign_k<W, 0, 0>(h, p_add, dump, meas);
+    if (tx == 8) return launch_assign_k<W, 8, 0>(h, p_add, dump, meas);
+    if (tx == 16) return launch_assign_k<W, 16, 0>(h, p_add, dump, meas);
+    return launch_assign_k<W, 32, 0>(h, p_add, dump, meas);
 }
 
 // measure: the assign phase also measures the spins it starts from (only where the block
@@ -290,32 +293,24 @@ int launch_assign(swb_lattice *h, float p_add, const AssignDump &dump = AssignDu
 
 int launch_merge(swb_lattice *h)
 {
-    const dim3 grid(h->g.nbx, h->g.nby);
-    k_merge<<<grid, h->g.BX + h->g.BY, 0, h->stream>>>(h->g, h->edge, h->labels, h->fault, h->linked);
-    SWB_LAUNCHED();
-    if (h->linked) {
-        k_resolve<<<grid, h->g.BX + h->g.BY, 0, h->stream>>>(h->g, h->linked, h->labels, h->fault);
-        SWB_LAUNCHED();
-    }
-    return SWB_OK;
+    return launch_next(early_launch(h), k_merge, dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream, h->g,
+                       h->edge, h->labels, h->fault, h->linked);
+}
+
+int launch_resolve(swb_lattice *h)
+{
+    if (!h->linked)
+        return SWB_OK;
+    return launch_next(early_launch(h), k_resolve, dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream, h->g,
+                       h->linked, h->labels, h->fault);
 }
 
 int launch_flip(swb_lattice *h, bool write_labels)
 {
-    const dim3 grid(h->g.nbx, h->g.nby);
-    if (h->linked) {
-        if (write_labels)
-            k_flip<true, true><<<grid, kFlipThreads, h->smem_flip, h->stream>>>(h->g, h->spins, h->labels, h->fault);
-        else
-            k_flip<false, true><<<grid, kFlipThreads, h->smem_flip, h->stream>>>(h->g, h->spins, h->labels, h->fault);
-    } else {
-        if (write_labels)
-            k_flip<true, false><<<grid, kFlipThreads, h->smem_flip, h->stream>>>(h->g, h->spins, h->labels, h->fault);
-        else
-            k_flip<false, false><<<grid, kFlipThreads, h->smem_flip, h->stream>>>(h->g, h->spins, h->labels, h->fault);
-    }
-    SWB_LAUNCHED();
-    return SWB_OK;
+    auto k = h->linked ? (write_labels ? k_flip<true, true> : k_flip<false, true>)
+                       : (write_labels ? k_flip<true, false> : k_flip<false, false>);
+    return launch_next(early_launch(h), k, dim3(h->g.nbx, h->g.nby), kFlipThreads, h->smem_flip, h->stream, h->g,
+                       h->spins, h->labels, h->fault);
 }
 
 int launch_sweep(swb_lattice *h, float p_add, bool write_labels, const AssignDump &dump = AssignDump{},
@@ -325,15 +320,15 @@ int launch_sweep(swb_lattice *h, float p_add, bool write_labels, const AssignDum
         return rc;
     if (int rc = launch_merge(h))
         return rc;
+    if (int rc = launch_resolve(h))
+        return rc;
     return launch_flip(h, write_labels);
 }
 
 int launch_measure(swb_lattice *h, int accumulate)
 {
-    k_measure<<<h->measure_grid, 256, 0, h->stream>>>(h->g.L0, h->g.L1, h->spins, h->obs, h->series, h->series_cap,
-                                                       accumulate);
-    SWB_LAUNCHED();
-    return SWB_OK;
+    return launch_next(early_launch(h), k_measure, h->measure_grid, 256, 0, h->stream, h->g.L0, h->g.L1, h->spins,
+                       h->obs, h->series, h->series_cap, accumulate);
 }
 
 // A measurement of the current spins that swb_sweep left for the next sweep's assign phase to
@@ -442,17 +437,18 @@ int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uin
         return fail(SWB_ERR_ARGUMENT, "unsupported tile %u x %u (tile_x in {8,16,32}, 2 <= tile_y <= 32)", tile_x, tile_y);
     if (!valid_width(lcg_width))
         return fail(SWB_ERR_ARGUMENT, "unsupported lcg32 width %u (8, 16 or 32)", lcg_width);
-    if (make_geo(L0, L1, tile_x, tile_y, lcg_width, kAssignThreads).nby > kMaxGridY)
+    if (make_geo(L0, L1, tile_x, tile_y).nby > kMaxGridY)
         return fail(SWB_ERR_ARGUMENT, "lattice of %u rows needs more than %u block rows", L1, kMaxGridY);
     swb_lattice *h = new swb_lattice();
     h->device = device;
     h->W = lcg_width;
     h->seed_base = seed_base;
-    h->g = make_geo(L0, L1, tile_x, tile_y, lcg_width, kAssignThreads);
+    h->g = make_geo(L0, L1, tile_x, tile_y);
     h->n = (size_t)L0 * L1;
     h->n_tiles = h->g.n0 * h->g.n1;
     h->n_blocks = h->g.nbx * h->g.nby;
-    h->smem_assign = assign_smem(h->g, h->W).total;
+    h->bands = assign_bands(h->g);
+    h->smem_assign = strip_smem(h->g, h->W, h->bands).total;
     auto cleanup = [&](int rc) {
         swb_destroy(h);
         return rc;
@@ -475,7 +471,7 @@ int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uin
     SWB_TRY(cudaMalloc(&h->rng_sel, (size_t)h->n_tiles * h->W));
     SWB_TRY(cudaMalloc(&h->rng_iter, (size_t)h->n_tiles * sizeof(uint32_t)));
     SWB_TRY(cudaMalloc(&h->edge, (size_t)h->n_blocks * kEdgeWords * sizeof(uint32_t)));
-    bool resolve = h->n_blocks >= kResolveMinBlocks || h->g.BX * h->g.BY >= kResolveBlockSites;
+    bool resolve = h->n >= kResolveMinSites;
     if (const char *e = std::getenv("SWB_RESOLVE_MIN_BLOCKS"))
         resolve = h->n_blocks >= (uint32_t)std::strtoul(e, nullptr, 10);
     if (resolve)
@@ -828,16 +824,12 @@ int swb_sweep_timed(swb_lattice *h, float temperature, uint32_t n_sweeps, int pe
         if ((rc = launch_assign(h, p_add)))
             break;
         SWB_CUDA(cudaEventRecord(ev[2], h->stream));
-        k_merge<<<dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream>>>(h->g, h->edge, h->labels, h->fault,
-                                                                               h->linked);
-        SWB_LAUNCHED();
+        if ((rc = launch_merge(h)))
+            break;
         SWB_CUDA(cudaEventRecord(ev[3], h->stream));
         // resolve + flip: the reference's ResolveLabels and FlipClusters
-        if (h->linked) {
-            k_resolve<<<dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream>>>(h->g, h->linked, h->labels,
-                                                                                     h->fault);
-            SWB_LAUNCHED();
-        }
+        if ((rc = launch_resolve(h)))
+            break;
         if ((rc = launch_flip(h, false)))
             break;
         SWB_CUDA(cudaEventRecord(ev[4], h->stream));
@@ -1055,17 +1047,18 @@ int swb_sweep_static(void *stream, uint32_t L0, uint32_t L1, uint32_t tile_x, ui
         return fail(SWB_ERR_ARGUMENT, "unsupported lcg32 width %u (8, 16 or 32)", lcg_width);
     if (!(temperature > 0.0f) || !std::isfinite(temperature))
         return fail(SWB_ERR_ARGUMENT, "temperature must be positive and finite");
-    if (make_geo(L0, L1, tile_x, tile_y, lcg_width, kAssignThreads).nby > kMaxGridY)
+    if (make_geo(L0, L1, tile_x, tile_y).nby > kMaxGridY)
         return fail(SWB_ERR_ARGUMENT, "lattice of %u rows needs more than %u block rows", L1, kMaxGridY);
 
     swb_lattice h;  // a view: caller's buffers plus the static scratch; owns nothing
     h.stream = static_cast<cudaStream_t>(stream);
     h.W = lcg_width;
-    h.g = make_geo(L0, L1, tile_x, tile_y, lcg_width, kAssignThreads);
+    h.g = make_geo(L0, L1, tile_x, tile_y);
     h.n = (size_t)L0 * L1;
     h.n_tiles = h.g.n0 * h.g.n1;
     h.n_blocks = h.g.nbx * h.g.nby;
-    h.smem_assign = assign_smem(h.g, h.W).total;
+    h.bands = assign_bands(h.g);
+    h.smem_assign = strip_smem(h.g, h.W, h.bands).total;
     h.smem_flip = flip_smem_bytes(h.g);
     const size_t labels_bytes = align256(h.n * sizeof(uint32_t) + 16);
     const size_t edge_bytes = align256((size_t)h.n_blocks * kEdgeWords * sizeof(uint32_t));
