@@ -45,6 +45,7 @@
 #include "../../include/swb200.h"
 #include "sw_core.cuh"
 #include "sw_strip.cuh"
+#include "sw_whole.cuh"
 
 namespace swb {
 
@@ -226,6 +227,7 @@ struct swb_lattice {
     unsigned int *fault = nullptr;  // set by a chase that exceeded kChainCap
     int measure_grid = 0;
     uint32_t smem_flip = 0;
+    Whole whole{};                 // plain sweeps run as one kernel (whole.ctas != 0)
     bool spins_attached = false;   // spins point at a caller-owned device buffer (swb_attach_spins)
     bool fused_measure = false;    // the assign phase can measure the spins it starts from
     bool measure_pending = false;  // a sample of the current spins is still to be taken
@@ -316,6 +318,10 @@ int launch_flip(swb_lattice *h, bool write_labels)
 int launch_sweep(swb_lattice *h, float p_add, bool write_labels, const AssignDump &dump = AssignDump{},
                  bool measure = false)
 {
+    if (h->whole.ctas && !write_labels)
+        return launch_whole(h->whole, h->W, h->spins, h->rng_state, h->rng_sel, h->rng_iter, accept_threshold(p_add),
+                            measure ? MeasureArgs{h->obs, h->series, h->series_cap} : MeasureArgs{}, h->fault,
+                            h->stream);
     if (int rc = launch_assign(h, p_add, dump, measure))
         return rc;
     if (int rc = launch_merge(h))
@@ -472,8 +478,17 @@ int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uin
     SWB_TRY(cudaMalloc(&h->rng_iter, (size_t)h->n_tiles * sizeof(uint32_t)));
     SWB_TRY(cudaMalloc(&h->edge, (size_t)h->n_blocks * kEdgeWords * sizeof(uint32_t)));
     bool resolve = h->n >= kResolveMinSites;
-    if (const char *e = std::getenv("SWB_RESOLVE_MIN_BLOCKS"))
+    h->whole = make_whole(L0, L1, tile_x, tile_y);
+    if (const char *e = std::getenv("SWB_RESOLVE_MIN_BLOCKS")) {
         resolve = h->n_blocks >= (uint32_t)std::strtoul(e, nullptr, 10);
+        h->whole.ctas = 0;
+    }
+    if (h->whole.ctas) {
+        bool fits = false;
+        SWB_TRY(allow_whole(h->whole, h->W, &fits));
+        if (!fits)
+            h->whole.ctas = 0;
+    }
     if (resolve)
         SWB_TRY(cudaMalloc(&h->linked, (size_t)h->n_blocks * (h->g.BX + h->g.BY) * sizeof(uint32_t)));
     SWB_TRY(cudaMalloc(&h->obs, sizeof(Obs)));
@@ -794,7 +809,7 @@ int swb_launches_per_sweep(swb_lattice *h, uint32_t *launches)
 {
     if (!h || !launches)
         return fail(SWB_ERR_ARGUMENT, "NULL argument");
-    *launches = h->linked ? 4 : 3;
+    *launches = h->whole.ctas ? 1 : h->linked ? 4 : 3;
     return SWB_OK;
 }
 

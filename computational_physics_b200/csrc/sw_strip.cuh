@@ -18,7 +18,7 @@
 // With many blocks a block is one band (4 warps: no seams between bands, and instruction issue is what
 // bounds it: 2.8 warp instructions per site, of which scan 0.8, draws 0.7, unions 0.5, labels 0.3, the
 // rest 0.5); with few, a band per tile row (up to 16 warps), which shortens every warp's serial walk.
-// 16384^2 with 16 x 8 tiles: 910 us a launch (1305 with staged spins, bond words through shared memory and
+// 16384^2 with 16 x 8 tiles: 890 us a launch (1305 with staged spins, bond words through shared memory and
 // a find per site).
 #pragma once
 
@@ -319,7 +319,6 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
         strip_stream<W, TXc, TYc>(g, bxi, byi, strip, trow0, trows, 0, rng_state, rng_sel, rng_iter);
     __syncthreads();
 
-    uint32_t listed = 0;  // unions in the piece's list
     if (ncols != 0) {
         strip_draws<W, TXc, TYc>(g, bxi, byi, strip, trow0, trows, first_tile, d, L.slots, pairs, rng_state, rng_sel,
                                  rng_iter, thr);
@@ -416,59 +415,55 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
             above = lab;
         }
         __syncwarp();
+    }
+    if (kEarly && ncols == 0)
+        after_previous();
+    __syncthreads();
 
-        // The unions: lane r lists the marked sites of row r, then the list is worked off one per
-        // lane (inside the scan they would run, divergent, on almost every row).  Each entry becomes
-        // the label its union hung below another (every label at most once), or none.
-        const uint32_t mine = lane < rows ? d[lane] : 0u;
-        uint32_t end = __popc(mine);  // inclusive prefix sum over the rows
+    // The unions, within the pieces and across them: lane r lists row r's marked sites (a band's first row:
+    // those bonded to the band above) and the bond from its last column into the next strip (unless the
+    // rows above join the same runs); then the list is worked off one entry per lane -- inside the scan
+    // they would run, divergent, on almost every row.  Each entry becomes the label its union hung below
+    // another (every label at most once), or none.
+    uint32_t listed = 0;
+    if (ncols != 0) {
+        uint32_t mine = lane < rows ? d[lane] : 0u, across = 0;
+        if (lane == 0 && band != 0) {
+            const uint2 up = last[-(int)nstrips];  // {y, x} bonds of the row above the piece
+            mine = up.x & ~((up.x & up.y & ~words[0].x) << 1);
+        }
+        if (ncols == 32 && xs + 32 < bxv && lane < rows) {
+            const uint4 a = words[lane], b = words[g.BY + lane];
+            const bool same = lane != 0 && (~words[lane - (lane != 0)].x & a.z) >> 31 && (b.z & 1u);
+            across = !(a.x >> 31) && !same;
+        }
+        __syncwarp();
+        uint32_t end = __popc(mine) + across;  // inclusive prefix sum over the rows
 #pragma unroll
         for (uint32_t o = 1; o < 32; o *= 2) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
             if (lane >= o)
                 end += v;
         }
-        const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
-        for (uint32_t b0 = 0; b0 == 0 || b0 < total; b0 += kStripList) {
+        listed = __shfl_sync(0xffffffffu, end, 31);
+        const uint32_t l0 = (r0 + lane) * kBlockPitch + xs;
+        for (uint32_t b0 = 0; b0 < listed; b0 += kStripList) {
             __syncwarp();
-            uint32_t k = end - __popc(mine) - b0;
+            uint32_t k = end - __popc(mine) - across - b0;
             for (uint32_t left = mine; left; left &= left - 1, ++k)
                 if (k < kStripList)  // unsigned: also false before the window
-                    d[k] = (r0 + lane) * kBlockPitch + xs + __ffs(left) - 1;
+                    d[k] = l0 + __ffs(left) - 1;
+            if (across && k < kStripList)
+                d[k] = kLocalFlag | (l0 + 31);
             __syncwarp();
-            const uint32_t n = min(total - b0, kStripList);
+            const uint32_t n = min(listed - b0, kStripList);
             for (uint32_t i = lane; i < n; i += 32) {
-                const uint32_t l = d[i];
-                d[i] = uf_union_link(parent, parent[l - kBlockPitch], parent[l]);
+                const uint32_t v = d[i], l = v & kLocalMask;
+                d[i] = uf_union_link(parent, parent[(v & kLocalFlag) ? l + 1 : l - kBlockPitch], parent[l]);
             }
         }
-        if (total > kStripList && lane == 0)
+        if (listed > kStripList && lane == 0)
             sums[2] = 1;  // the list no longer holds every linked label
-        listed = total;
-    }
-    if (kEarly && ncols == 0)
-        after_previous();
-    __syncthreads();
-
-    // Join the pieces: x-bonds from a strip's last column into the next strip, one row per lane
-    // (skipping those whose upper neighbour already joins the same runs), and y-bonds into the band
-    // below, one column per lane.
-    uint32_t joined = kNoLink;
-    if (ncols == 32 && xs + 32 < bxv && lane < rows) {
-        const uint4 a = words[lane], b = words[g.BY + lane];
-        const bool same = lane != 0 && (~words[lane - (lane != 0)].x & a.z) >> 31 && (b.z & 1u);
-        if (!(a.x >> 31) && !same) {
-            const uint32_t l = (r0 + lane) * kBlockPitch + xs + 31;
-            joined = uf_union_link(parent, parent[l], parent[l + 1]);
-        }
-    }
-    if (ncols != 0 && band != 0) {
-        const uint2 up = last[-(int)nstrips];  // {y, x} bonds of the row above the piece
-        const uint32_t U = up.x & ~((up.x & up.y & ~words[0].x) << 1);
-        if ((U >> lane) & 1u) {
-            const uint32_t l = r0 * kBlockPitch + xs + lane;
-            uf_union_link(parent, parent[l - kBlockPitch], parent[l]);
-        }
     }
     if (threadIdx.x == 0)
         eblk[0] = reinterpret_cast<const uint32_t *>(sums)[3];
@@ -479,8 +474,6 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
     // block in bands skips this pass and its barrier: its few sites per thread walk to their roots.
     bool deep = bands != 1;
     if (!deep) {
-        if (joined != kNoLink)
-            uf_flatten(parent, joined);
         for (uint32_t i = lane; i < min(listed, kStripList); i += 32) {
             const uint32_t b = d[i];
             if (b != kNoLink)

@@ -55,9 +55,10 @@ uint64_t swb_kernel_launches(void);
  * the top bit used internally).  tile_x in {8, 16, 32},
  * 2 <= tile_y <= 32, lcg_width in {8, 16, 32}.  Spins start all 0.  A lattice of
  * at least 2048 x 2048 sites resolves merged roots in a kernel of their own before the flip,
- * others in the flip; the environment variable
- * SWB_RESOLVE_MIN_BLOCKS, read here, replaces that rule by a block count.  Both forms give
- * identical results. */
+ * others in the flip; lattices small enough for one thread-block cluster (up to about 512 x 256
+ * sites) run a whole sweep in one kernel.  The environment variable SWB_RESOLVE_MIN_BLOCKS, read
+ * here, replaces the first rule by a block count and switches the one-kernel form off.  All forms
+ * give identical results. */
 int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uint32_t tile_y,
                uint32_t lcg_width, uint32_t seed_base, int device);
 
@@ -107,7 +108,8 @@ int swb_sweep(swb_lattice *h, float temperature, uint32_t n_sweeps, uint32_t mea
 int swb_sweep_recorded(swb_lattice *h, float temperature, uint8_t *bonds, uint32_t *labels_assign,
                        uint32_t *labels_final);
 
-/* One sweep through the same kernels swb_sweep runs, with their dumps switched on, to HOST
+/* One sweep through the phase kernels of swb_sweep (which runs lattices that fit one thread-block
+ * cluster in one kernel instead, with identical results), with their dumps switched on, to HOST
  * buffers (each may be NULL): bonds (as swb_sweep_recorded), labels_block = the minimum global
  * site index of each site's component over the bonds inside its block (swb_geometry gives the
  * block shape; bonds across block edges and the periodic wrap are left to the merge), and the
