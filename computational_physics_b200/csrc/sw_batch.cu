@@ -29,7 +29,6 @@
 namespace swb {
 
 constexpr uint32_t kMeasureThreads = 256;      // measure: one thread per 16 sites of a 4096-site chunk
-constexpr uint32_t kMergeThreads = 160;        // merge, resolve: one thread per block edge site (BX + BY <= 160)
 constexpr uint32_t kFlipThreads = 256;         // flip: four quads of a 128 x 32 block per thread
 constexpr uint32_t kChunkSites = 4096;         // measure work item
 constexpr uint32_t kRoundGroups = 2;           // lattice groups whose sweeps run side by side in a round
@@ -137,30 +136,33 @@ __global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) kb_assign(BatchL
     }
 }
 
+// kWarps warps per item (merge_warps).
+template <uint32_t kWarps>
 __global__ void __launch_bounds__(kMergeThreads) kb_merge(const BatchLat *lats, const BlockRec *recs,
                                                           const uint32_t total, unsigned int *fault)
 {
+    __shared__ uint8_t list[kMergeThreads / 32][kMergeList];
+    const uint32_t i = (blockIdx.x * kMergeThreads + threadIdx.x) / 32, item = i / kWarps;
     after_previous();
-    for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    if (item < total) {
         const BlockRec r = recs[item];
-        const Geo g = rec_geo(r);
         const bool active = lats[r.lat].sweeps_left != 0;
-        if (threadIdx.x < g.BX + g.BY)
-            merge_block(g, r.bxy & 0xFFFFu, r.bxy >> 16, threadIdx.x, r.edge, r.labels, fault, r.linked, active);
+        merge_block<kWarps>(rec_geo(r), r.bxy & 0xFFFFu, r.bxy >> 16, i % kWarps, r.edge, r.labels, fault, r.linked,
+                            list[threadIdx.x / 32], active);
     }
 }
 
 // ResolveLabels for the roots each block's merge linked (resolve_block).
+template <uint32_t kWarps>
 __global__ void __launch_bounds__(kMergeThreads) kb_resolve(const BatchLat *lats, const BlockRec *recs,
                                                             const uint32_t total, unsigned int *fault)
 {
+    const uint32_t i = (blockIdx.x * kMergeThreads + threadIdx.x) / 32, item = i / kWarps;
     after_previous();
-    for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    if (item < total) {
         const BlockRec r = recs[item];
-        const Geo g = rec_geo(r);
         const bool active = lats[r.lat].sweeps_left != 0;
-        if (threadIdx.x < g.BX + g.BY)
-            resolve_block(g, r.bxy & 0xFFFFu, r.bxy >> 16, threadIdx.x, r.linked, r.labels, fault, active);
+        resolve_block<kWarps>(rec_geo(r), r.bxy & 0xFFFFu, r.bxy >> 16, i % kWarps, r.linked, r.labels, fault, active);
     }
 }
 
@@ -406,7 +408,7 @@ uint64_t lattice_bytes(const Geo &g, uint32_t W, uint64_t series_cap)
     const uint64_t n = (uint64_t)g.L0 * g.L1, tiles = (uint64_t)g.n0 * g.n1, blocks = (uint64_t)g.nbx * g.nby;
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     return al(n) + al(4 * n) + al(4 * tiles * W) + al(tiles * W) + al(4 * tiles) + al(4 * kEdgeWords * blocks) +
-           al(4 * (uint64_t)(g.BX + g.BY) * blocks) + al(sizeof(Obs)) + al(16 * series_cap);
+           al(4 * (uint64_t)kMergeSlots * blocks) + al(sizeof(Obs)) + al(16 * series_cap);
 }
 
 int upload_descriptor(swb_batch *b, uint32_t id)
@@ -567,7 +569,9 @@ int launch_assign_b(swb_batch *b, const uint2 *items, uint32_t n, cudaStream_t s
 
 int launch_merge_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_t st, bool early)
 {
-    return launch_next(early, kb_merge, std::max(n, 1u), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault);
+    const uint32_t w = merge_warps(n);
+    auto k = w == kEdgeParts ? kb_merge<kEdgeParts> : w == 1 ? kb_merge<1> : kb_merge<kMidWarps>;
+    return launch_next(early, k, merge_grid(n), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault);
 }
 
 // kb_resolve, where the launch has one (few items: the flip chases the merged roots, as in swb_create).
@@ -575,7 +579,9 @@ int launch_resolve_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_
 {
     if (n < kResolveItems)
         return SWB_OK;
-    return launch_next(early, kb_resolve, std::max(n, 1u), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault);
+    const uint32_t w = merge_warps(n);
+    auto k = w == kEdgeParts ? kb_resolve<kEdgeParts> : w == 1 ? kb_resolve<1> : kb_resolve<kMidWarps>;
+    return launch_next(early, k, merge_grid(n), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault);
 }
 
 int launch_flip_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_t st, bool early)
@@ -871,7 +877,7 @@ int swb_batch_add(swb_batch *b, uint32_t L0, uint32_t L1, uint32_t tile_x, uint3
     d.rng_sel = reinterpret_cast<uint8_t *>(p); p += al(tiles * b->W);
     d.rng_iter = reinterpret_cast<uint32_t *>(p); p += al(4 * tiles);
     d.edge = reinterpret_cast<uint32_t *>(p); p += al(4 * kEdgeWords * blocks);
-    d.linked = reinterpret_cast<uint32_t *>(p); p += al(4 * (uint64_t)(g.BX + g.BY) * blocks);
+    d.linked = reinterpret_cast<uint32_t *>(p); p += al(4 * (uint64_t)kMergeSlots * blocks);
     d.obs = reinterpret_cast<Obs *>(p); p += al(sizeof(Obs));
     d.series = reinterpret_cast<long long *>(p);
     d.series_cap = b->series_cap;

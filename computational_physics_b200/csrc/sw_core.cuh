@@ -141,7 +141,15 @@ struct U32 {  // a compile-time uint32_t passed as a value
 };
 
 constexpr uint32_t kMaxGridY = 65535;  // block rows of a lattice: the kernels' grid y
-constexpr uint32_t kEdgeWords = 8;  // per block: [0] right edge rows, [1..4] bottom edge columns
+// Edge words of a block: what its merge needs.  [0] bonds out of the last column (a bit per row), [1..4] out
+// of the last row (a bit per column); then, to leave out bonds that join the same two runs as the bond
+// before them: [5] y-bonds in the last column, [6] in the first column (a bit per row), [7..10] x-bonds in
+// the last row, [11..14] in the first row.  A recorded sweep leaves [5..14] zero: nothing is left out.
+constexpr uint32_t kEdgeWords = 16;
+constexpr uint32_t kEdgeYLast = 5, kEdgeYFirst = 6, kEdgeXLast = 7, kEdgeXFirst = 11;
+constexpr uint32_t kEdgeParts = 5;       // words [0..4]
+constexpr uint32_t kMergeList = kEdgeParts * 32;  // edge bonds of a block, at most
+constexpr uint32_t kMergeThreads = 160;  // merge, resolve: one warp or several per block
 
 // Label encoding between the assign and flip phases of a sweep.  A block root holds its global
 // site index (< 2^31); these are the only entries the merge reads and links.  Every other site
@@ -575,61 +583,129 @@ __device__ __forceinline__ void assign_block_tiles(const Geo &g, const uint32_t 
         edge[((size_t)byi * g.nbx + bxi) * kEdgeWords + tid] = edge_s[tid];
 }
 
-// Unions across the right and bottom edge (periodic) of block (bxi, byi): thread t < BY takes
-// row t of the right edge, BY <= t < BY + BX column t - BY of the bottom edge.  With `linked`,
-// slot t of the block's BX + BY slots receives the root this thread's union linked (kNoLink
-// for none): every block root the merge turns into a non-root appears in exactly one slot.
-// With active false (a lattice whose sweep budget is spent) nothing is written; the edge words
-// are read all the same, so their load need not wait for the budget's.
-__device__ __forceinline__ void merge_block(const Geo &g, const uint32_t bxi, const uint32_t byi, const uint32_t t,
-                                            const uint32_t *edge, uint32_t *labels, unsigned int *fault,
-                                            uint32_t *linked, const bool active = true)
+constexpr uint32_t kMidWarps = 3;
+
+// Warps per block in merge and resolve: one per edge word while the blocks leave the GPU's warps free, fewer
+// with lists beyond.  Measured with 1 / 2 / 3 / 4 listing warps: 16384^2 sweep 1354 / 1360 / 1377 / 1386 us (a
+// thread per edge site: 1418); 4096^2 at T = 2.0 132.7 / 132.8 / 127.3 / 126.2, at T = 3.0 97.3 / 94.0 / 97.4 /
+// 98.3; 512-lattice mix round 269.6 / 269.7 / 267.5 / 270.3; 16 lattices 35.7 / 32.9 / 30.6 / 30.2 (by edge
+// site 29.0).
+inline uint32_t merge_warps(uint32_t blocks) { return blocks < 4096 ? kEdgeParts : blocks < 16384 ? kMidWarps : 1; }
+inline uint32_t merge_grid(uint32_t blocks)
 {
-    const uint32_t x0 = bxi * g.BX, y0 = byi * g.BY;
-    const uint32_t bxv = min(g.BX, g.L0 - x0), byv = min(g.BY, g.L1 - y0);
-    const uint32_t *e = edge + ((size_t)byi * g.nbx + bxi) * kEdgeWords;
-    size_t s = 0, nb = 0;
-    uint32_t nbx = bxi, nby = byi;  // block of the neighbour site
-    bool go = false;
-    if (t < g.BY) {
-        if (t < byv && ((e[0] >> t) & 1u)) {
-            s = (size_t)(y0 + t) * g.L0 + x0 + bxv - 1;
-            nb = (size_t)(y0 + t) * g.L0 + (x0 + bxv < g.L0 ? x0 + bxv : 0u);
-            nbx = bxi + 1 == g.nbx ? 0 : bxi + 1;
-            go = true;
-        }
-    } else {
-        const uint32_t xl = t - g.BY;
-        if (xl < bxv && ((e[1 + (xl >> 5)] >> (xl & 31)) & 1u)) {
-            s = (size_t)(y0 + byv - 1) * g.L0 + x0 + xl;
-            nb = (size_t)(y0 + byv < g.L1 ? y0 + byv : 0u) * g.L0 + x0 + xl;
-            nby = byi + 1 == g.nby ? 0 : byi + 1;
-            go = true;
-        }
-    }
-    uint32_t link = kNoLink;
-    if (go && active) {
-        const volatile uint32_t *vl = labels;
-        const uint32_t a = label_global(g, bxi, byi, vl[s]), b = label_global(g, nbx, nby, vl[nb]);
-        if (a != b)
-            link = guf_union_pair(labels, a, b, g.L0 * g.L1, fault);
-    }
-    if (linked && active)
-        linked[((size_t)byi * g.nbx + bxi) * (g.BX + g.BY) + t] = link;
+    constexpr uint32_t kWarps = kMergeThreads / 32;
+    const uint32_t n = (blocks * merge_warps(blocks) + kWarps - 1) / kWarps;
+    return n ? n : 1;
 }
 
-// ResolveLabels for the roots the merge linked (slot t of block (bxi, byi), after every merge
-// of the sweep): the root's chain is walked to the cluster's root, which is stored in its
-// label.  Afterwards every block root's label is its cluster's root, so the flip needs no
-// chase; the chases of all blocks are in flight together here instead of behind each flip
-// CTA's barrier.
-__device__ __forceinline__ void resolve_block(const Geo &g, const uint32_t bxi, const uint32_t byi, const uint32_t t,
-                                              const uint32_t *linked, uint32_t *labels,
-                                              unsigned int *fault, const bool active = true)
+// Merge slots of a block: the root that each edge bond's union linked (kNoLink for none) -- by edge site, or
+// with lists by their order and their number after the last; a multiple of 32 bytes.
+constexpr uint32_t kMergeSlots = kMergeList + 8;
+
+// Unions across the right and bottom edge (periodic) of block (bxi, byi), by warp `sub` of the kWarps
+// that share the block.  With many blocks each warp lists the edge bonds that may join two clusters (at
+// the critical temperature about a third of the edge sites: a thread per edge site left two lanes of
+// three idle through the label loads and walks), then takes its share, one per lane; with kEdgeParts
+// warps each takes one edge word as it is, the shorter way.  With `linked`, every block
+// root the merge turns into a non-root appears in exactly one of its slots.  With active false (a
+// lattice whose sweep budget is spent) nothing is written; the edge words are read all the same, so
+// their load need not wait for the budget's.
+template <uint32_t kWarps>
+__device__ __forceinline__ void merge_block(const Geo &g, const uint32_t bxi, const uint32_t byi, const uint32_t sub,
+                                            const uint32_t *edge, uint32_t *labels, unsigned int *fault,
+                                            uint32_t *linked, uint8_t *list, const bool active = true)
 {
-    const uint32_t b = linked[((size_t)byi * g.nbx + bxi) * (g.BX + g.BY) + t];
-    if (b != kNoLink && active)
-        labels[b] = guf_find(labels, b, g.L0 * g.L1, fault);  // the tree's minimum: other finds' atomicMin never undo it
+    const uint32_t lane = threadIdx.x & 31, under = (1u << lane) - 1u;
+    const uint32_t x0 = bxi * g.BX, y0 = byi * g.BY;
+    const uint32_t bxv = min(g.BX, g.L0 - x0), byv = min(g.BY, g.L1 - y0);
+    const uint32_t right = bxi + 1 == g.nbx ? 0 : bxi + 1, below = byi + 1 == g.nby ? 0 : byi + 1;
+    const size_t blk = (size_t)byi * g.nbx + bxi;
+    const uint32_t *e = edge + blk * kEdgeWords, *er = edge + ((size_t)byi * g.nbx + right) * kEdgeWords;
+    const uint32_t *eb = edge + ((size_t)below * g.nbx + bxi) * kEdgeWords;
+    uint32_t *slots = linked ? linked + blk * kMergeSlots : nullptr;
+    // the bonds of edge word w, and of those the ones whose next neighbour would join the same runs
+    auto part = [&](const uint32_t w, uint32_t &T) -> uint32_t {
+        if (w == 0) {
+            const uint32_t A = e[0];
+            T = A & e[kEdgeYLast] & er[kEdgeYFirst];
+            return A;
+        }
+        if ((w - 1) * 32 < bxv) {
+            const uint32_t A = e[w];
+            T = A & e[kEdgeXLast - 1 + w] & eb[kEdgeXFirst - 1 + w];
+            return A;
+        }
+        T = 0;
+        return 0;
+    };
+    auto unite = [&](const uint32_t i, const uint32_t t) {  // the i-th listed bond, edge site t
+        uint32_t s, nb, nbx = bxi, nby = byi;               // the site, its neighbour, the neighbour's block
+        if (t < 32) {
+            s = (y0 + t) * g.L0 + x0 + bxv - 1;
+            nb = (y0 + t) * g.L0 + (x0 + bxv < g.L0 ? x0 + bxv : 0u);
+            nbx = right;
+        } else {
+            s = (y0 + byv - 1) * g.L0 + x0 + t - 32;
+            nb = (y0 + byv < g.L1 ? y0 + byv : 0u) * g.L0 + x0 + t - 32;
+            nby = below;
+        }
+        const volatile uint32_t *vl = labels;
+        const uint32_t a = label_global(g, bxi, byi, vl[s]), b = label_global(g, nbx, nby, vl[nb]);
+        const uint32_t link = a != b ? guf_union_pair(labels, a, b, g.L0 * g.L1, fault) : kNoLink;
+        if (slots)
+            slots[i] = link;
+    };
+    if constexpr (kWarps == kEdgeParts) {
+        uint32_t T;
+        const uint32_t A = part(sub, T), U = A & ~(T << 1);
+        if (!active)
+            return;
+        if ((U >> lane) & 1u)
+            unite(sub * 32 + lane, sub * 32 + lane);
+        else if (slots)
+            slots[sub * 32 + lane] = kNoLink;
+        return;
+    }
+    uint32_t T = 0, n = 0;
+    const uint32_t A = lane < kEdgeParts ? part(lane, T) : 0u;
+    const uint32_t carry = __shfl_up_sync(0xffffffffu, T, 1) >> 31;
+    const uint32_t U = A & ~(T << 1 | (lane < 2 ? 0u : carry));
+#pragma unroll
+    for (uint32_t w = 0; w < kEdgeParts; ++w) {
+        const uint32_t word = __shfl_sync(0xffffffffu, U, w);
+        if ((word >> lane) & 1u)
+            list[n + __popc(word & under)] = (uint8_t)(w * 32 + lane);
+        n += __popc(word);
+    }
+    __syncwarp();
+    if (!active)
+        return;
+    if (slots && lane == 0 && sub == 0)
+        slots[kMergeList] = n;
+    for (uint32_t i = sub * 32 + lane; i < n; i += kWarps * 32)
+        unite(i, list[i]);
+}
+
+// ResolveLabels for the roots the merge linked (block (bxi, byi)'s slots, after every merge of the sweep):
+// the root's chain is walked to the cluster's root, which is stored in its label.  Afterwards every
+// block root's label is its cluster's root, so the flip needs no chase; the chases of all blocks are
+// in flight together here instead of behind each flip CTA's barrier.
+template <uint32_t kWarps>
+__device__ __forceinline__ void resolve_block(const Geo &g, const uint32_t bxi, const uint32_t byi, const uint32_t sub,
+                                              const uint32_t *linked, uint32_t *labels, unsigned int *fault,
+                                              const bool active = true)
+{
+    const uint32_t *slots = linked + ((size_t)byi * g.nbx + bxi) * kMergeSlots;
+    uint32_t i = sub * 32 + (threadIdx.x & 31);
+    uint32_t b = slots[i];
+    const uint32_t n = !active ? 0u : kWarps == kEdgeParts ? kMergeList : min(slots[kMergeList], kMergeList);
+    while (i < n) {
+        if (b != kNoLink)
+            labels[b] = guf_find(labels, b, g.L0 * g.L1, fault);  // the tree's minimum: other finds' atomicMin never undo it
+        i += kWarps * 32;
+        if (i < n)
+            b = slots[i];
+    }
 }
 
 // Shared memory of flip_block: the resolved label of every block root.

@@ -104,19 +104,27 @@ __global__ void __launch_bounds__(kTilesThreads) k_assign_tiles(const Geo g, con
     assign_block_tiles<W>(g, blockIdx.x, blockIdx.y, spins, labels, rng_state, rng_sel, rng_iter, thr, edge, dump, smem);
 }
 
-__global__ void __launch_bounds__(256) k_merge(const Geo g, const uint32_t *edge, uint32_t *labels, unsigned int *fault,
-                                               uint32_t *linked)
+// kWarps warps per block (merge_warps).
+template <uint32_t kWarps>
+__global__ void __launch_bounds__(kMergeThreads) k_merge(const Geo g, const uint32_t *edge, uint32_t *labels,
+                                                         unsigned int *fault, uint32_t *linked)
 {
+    __shared__ uint8_t list[kMergeThreads / 32][kMergeList];
+    const uint32_t i = (blockIdx.x * kMergeThreads + threadIdx.x) / 32, blk = i / kWarps, byi = blk / g.nbx;
     after_previous();
-    merge_block(g, blockIdx.x, blockIdx.y, threadIdx.x, edge, labels, fault, linked);
+    if (byi < g.nby)
+        merge_block<kWarps>(g, blk - byi * g.nbx, byi, i % kWarps, edge, labels, fault, linked, list[threadIdx.x / 32]);
 }
 
-// The linked roots of one block's merge slots (resolve_block), one thread per slot.
-__global__ void __launch_bounds__(256) k_resolve(const Geo g, const uint32_t *linked, uint32_t *labels,
-                                                 unsigned int *fault)
+// The linked roots of the blocks' merge slots (resolve_block).
+template <uint32_t kWarps>
+__global__ void __launch_bounds__(kMergeThreads) k_resolve(const Geo g, const uint32_t *linked, uint32_t *labels,
+                                                           unsigned int *fault)
 {
+    const uint32_t i = (blockIdx.x * kMergeThreads + threadIdx.x) / 32, blk = i / kWarps, byi = blk / g.nbx;
     after_previous();
-    resolve_block(g, blockIdx.x, blockIdx.y, threadIdx.x, linked, labels, fault);
+    if (byi < g.nby)
+        resolve_block<kWarps>(g, blk - byi * g.nbx, byi, i % kWarps, linked, labels, fault);
 }
 
 // Resolve + flip, one CTA per block (flip_block).
@@ -295,16 +303,20 @@ int launch_assign(swb_lattice *h, float p_add, const AssignDump &dump = AssignDu
 
 int launch_merge(swb_lattice *h)
 {
-    return launch_next(early_launch(h), k_merge, dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream, h->g,
-                       h->edge, h->labels, h->fault, h->linked);
+    const uint32_t w = merge_warps(h->n_blocks);
+    auto k = w == kEdgeParts ? k_merge<kEdgeParts> : w == 1 ? k_merge<1> : k_merge<kMidWarps>;
+    return launch_next(early_launch(h), k, merge_grid(h->n_blocks), kMergeThreads, 0, h->stream, h->g, h->edge, h->labels,
+                       h->fault, h->linked);
 }
 
 int launch_resolve(swb_lattice *h)
 {
     if (!h->linked)
         return SWB_OK;
-    return launch_next(early_launch(h), k_resolve, dim3(h->g.nbx, h->g.nby), h->g.BX + h->g.BY, 0, h->stream, h->g,
-                       h->linked, h->labels, h->fault);
+    const uint32_t w = merge_warps(h->n_blocks);
+    auto k = w == kEdgeParts ? k_resolve<kEdgeParts> : w == 1 ? k_resolve<1> : k_resolve<kMidWarps>;
+    return launch_next(early_launch(h), k, merge_grid(h->n_blocks), kMergeThreads, 0, h->stream, h->g, h->linked,
+                       h->labels, h->fault);
 }
 
 int launch_flip(swb_lattice *h, bool write_labels)
@@ -490,7 +502,7 @@ int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uin
             h->whole.ctas = 0;
     }
     if (resolve)
-        SWB_TRY(cudaMalloc(&h->linked, (size_t)h->n_blocks * (h->g.BX + h->g.BY) * sizeof(uint32_t)));
+        SWB_TRY(cudaMalloc(&h->linked, (size_t)h->n_blocks * kMergeSlots * sizeof(uint32_t)));
     SWB_TRY(cudaMalloc(&h->obs, sizeof(Obs)));
     h->series_cap = 1ull << 17;  // 131072 measurements (2 MiB)
     SWB_TRY(cudaMalloc(&h->series, h->series_cap * 2 * sizeof(long long)));

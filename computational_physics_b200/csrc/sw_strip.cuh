@@ -51,8 +51,8 @@ __host__ __device__ inline StripSmem strip_smem(const Geo &g, uint32_t W, uint32
     s.words = g.BY * kBlockPitch * 4;                  // [strip][BY] row words (below)
     s.last = s.words + ns * g.BY * 16;                 // [band][strip] {y, x} bonds of the piece's last row
     s.draws = s.last + ns * bands * 8;                 // [band][strip][dcap]
-    s.sums = s.draws + ns * bands * s.dcap * 4;        // energy and magnetisation sums, deep flag, right edge
-    s.pairs = s.sums + 16;                             // the five (a, c) pairs of lcg32
+    s.sums = s.draws + ns * bands * s.dcap * 4;        // energy and magnetisation sums, deep flag, edge words 0, 5, 6
+    s.pairs = s.sums + 32;                             // the five (a, c) pairs of lcg32
     s.total = s.pairs + 40;
     return s;
 }
@@ -310,10 +310,9 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
     uint2 *pairs = reinterpret_cast<uint2 *>(smem + L.pairs);
     if (threadIdx.x < 5) {
         pairs[threadIdx.x] = make_uint2(lcg_param_a(threadIdx.x), lcg_param_c(threadIdx.x));
-        if (threadIdx.x < 4)
-            sums[threadIdx.x] = 0;
     }
-
+    if (threadIdx.x < 6)
+        sums[threadIdx.x] = 0;
     const uint32_t trow0 = band * tpb, trows = ncols ? min(tpb, g.TBY - trow0) : 0;
     const StripTile first_tile =
         strip_stream<W, TXc, TYc>(g, bxi, byi, strip, trow0, trows, 0, rng_state, rng_sel, rng_iter);
@@ -356,9 +355,13 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
             Y = ~dy & AY & colm;
             if (lane + 1 == rows) {
                 *last = make_uint2(Y, X);
-                if (r0 + rows == byv)
+                if (r0 + rows == byv) {
                     eblk[1 + strip] = Y;  // bonds out of the block's last row
+                    eblk[kEdgeXLast + strip] = X;
+                }
             }
+            if (r0 + lane == 0)
+                eblk[kEdgeXFirst + strip] = X;
         }
         // Row words: the gaps ~X; the first y-bond up or run end from a run's start is the run's first
         // set bit of the second (bit 31 always ends a strip run); the bonds Yu to the row above; and of
@@ -372,10 +375,18 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
             if (lane < rows)
                 words[lane] = make_uint4(~X, Yu | ~X | 0x80000000u, Yu, Yu & ~((Yu & X & Xu) << 1));
         }
-        if (xs + 32 >= bxv) {  // bonds out of the block's last column
+        if (xs + 32 >= bxv) {  // bonds out of the block's last column, and along it
             const uint32_t e = __ballot_sync(0xffffffffu, (X >> (ncols - 1)) & 1u);
-            if (lane == 0)
+            const uint32_t yl = __ballot_sync(0xffffffffu, (Y >> (ncols - 1)) & 1u);
+            if (lane == 0) {
                 atomicOr(reinterpret_cast<unsigned int *>(sums) + 3, e << r0);
+                atomicOr(reinterpret_cast<unsigned int *>(sums) + 4, yl << r0);
+            }
+        }
+        if (strip == 0) {
+            const uint32_t yf = __ballot_sync(0xffffffffu, Y & 1u);
+            if (lane == 0)
+                atomicOr(reinterpret_cast<unsigned int *>(sums) + 5, yf << r0);
         }
         if constexpr (kMeasure) {  // s (s_right + s_down) and s: +1 per equal pair, -1 per unequal one
             int e = 0, m = 0;
@@ -465,8 +476,8 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
         if (listed > kStripList && lane == 0)
             sums[2] = 1;  // the list no longer holds every linked label
     }
-    if (threadIdx.x == 0)
-        eblk[0] = reinterpret_cast<const uint32_t *>(sums)[3];
+    if (threadIdx.x < 3)
+        eblk[threadIdx.x == 0 ? 0 : kEdgeYLast - 1 + threadIdx.x] = (uint32_t)sums[3 + threadIdx.x];
     __syncthreads();
 
     // Point every linked label straight at its root (they are the only labels that are not roots), so
