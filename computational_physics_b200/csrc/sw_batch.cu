@@ -2,13 +2,12 @@
 // tiles and temperatures advance together, one kernel launch per sweep phase for all of them.
 //
 // Work items.  Every active lattice contributes its blocks (TBX x TBY tiles) to one flat list
-// of block items (lattice slot, block coordinates), big lattices first.  kb_assign, kb_merge,
-// kb_resolve and kb_flip run one CTA per item (a CTA takes items blockIdx.x, blockIdx.x + gridDim.x, ...,
-// loading the next item's descriptor while it works on the current one, so a smaller grid
-// also covers the list); kb_measure pulls chunks of 4096 sites from a device counter
-// (atomicAdd), which the round's first kb_assign resets.  A sweep needs no host work and is one CUDA graph: the
-// lattices split into two groups (few items: one) whose phase kernels run on two streams side by side; the
-// graph is captured once and replayed, and captured again when the lattice set changes.
+// of block items (lattice slot, block coordinates), big lattices first.  kb_assign and kb_flip run one CTA
+// per item, kb_merge and kb_resolve one warp or several; kb_measure pulls chunks of 4096 sites from a
+// device counter (atomicAdd), which the next round empties.  A sweep needs no host work: with many items it is
+// one CUDA graph, the lattices in two groups whose phase kernels run on two streams side by side; the
+// graph is captured once and replayed, and captured again when the lattice set changes.  Few items are one
+// group, a chain of kernels launched early (launch_next).
 //
 // Per lattice the device keeps spins, labels, lcg32 streams (one per tile, seeded
 // seed_base + tile id as the reference's CPU path with one stream per tile), a sweep budget
@@ -19,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <vector>
@@ -55,6 +55,7 @@ struct BatchLat {
     unsigned long long series_cap;
     uint32_t thr;             // bond accept threshold, accept_threshold(p_add)
     uint32_t sweeps_left;     // sweeps still to run (kUnlimited: no limit)
+    uint32_t active;          // swept in the current round (set by its assign phase)
     uint32_t measure_every;   // measure after every measure_every-th sweep (0: never)
     uint32_t sweeps_done;     // sweeps completed
     uint32_t measure_base;    // first entry of this lattice's chunks in the round's measure list
@@ -62,9 +63,9 @@ struct BatchLat {
 
 struct BatchCounters {
     unsigned int measure_next;    // next entry of the measure list (device work counter)
+    unsigned int measure_chunks;  // entries of this round's measure list
     unsigned int n_active;        // lattices in the work lists
     unsigned int total_chunks;    // measure chunks of all active lattices (the list's capacity)
-    unsigned int measure_chunks;  // entries of this round's measure list
 };
 
 __device__ __forceinline__ uint32_t next_item(unsigned int *queue, uint32_t *slot)
@@ -109,44 +110,80 @@ __device__ __forceinline__ Geo rec_geo(const BlockRec &r)
     return g;
 }
 
-// With ctr (the first assign of a round) the measure list of the previous round is emptied.
+// Budgets change between a round's merge and the next round's assign (close_round), so the draws and the
+// choice of the lattices to sweep may run beside the previous round's last kernel.  With ctr (the first
+// assign of a round) the measure list of the previous round is emptied.
 template <int W, bool kAllShapes>
 __global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) kb_assign(BatchLat *lats, const uint2 *items,
                                                                           const uint32_t total, const uint32_t bands,
                                                                           BatchCounters *ctr)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    uint2 d = load_item(items, blockIdx.x, total);
-    after_previous();
-    if (ctr && blockIdx.x == 0 && threadIdx.x == 0) {
-        ctr->measure_next = 0;
-        ctr->measure_chunks = 0;
+    const uint2 d = load_item(items, blockIdx.x, total);
+    BatchLat *L = lats + d.x;
+    const bool on = blockIdx.x < total && L->sweeps_left != 0;
+    if (on) {
+        const Geo g = L->g;
+        assign_strips_any<W, false, false, true, kAllShapes>(g, d.y & 0xFFFFu, d.y >> 16, bands, L->spins, L->labels,
+                                                             L->rng_state, L->rng_sel, L->rng_iter, L->thr, L->edge,
+                                                             AssignDump{}, MeasureArgs{}, smem);
+    } else {
+        after_previous();
     }
-    for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
-        const uint2 next = load_item(items, item + gridDim.x, total);
-        const BatchLat *L = lats + d.x;
-        if (L->sweeps_left != 0) {
-            const Geo g = L->g;
-            assign_strips_any<W, false, false, false, kAllShapes>(g, d.y & 0xFFFFu, d.y >> 16, bands, L->spins,
-                                                                  L->labels, L->rng_state, L->rng_sel, L->rng_iter,
-                                                                  L->thr, L->edge, AssignDump{}, MeasureArgs{}, smem);
-            __syncthreads();
+    if (threadIdx.x == 0) {
+        if (blockIdx.x < total)
+            L->active = on;
+        if (ctr && blockIdx.x == 0) {
+            ctr->measure_next = 0;
+            ctr->measure_chunks = 0;
         }
-        d = next;
     }
 }
 
-// kWarps warps per item (merge_warps).
+// Bookkeeping of a round for lattices active[first .. first + n), after their assign phase: each lattice
+// that is swept counts the sweep and spends one from its budget; with chunk_lat (a round that measures)
+// every lattice due for a sample (measure_every divides its sweep count) appends its 4096-site chunks to
+// the round's measure list, so kb_measure visits only those.  Called by `threads` threads, this one `t`.
+__device__ __forceinline__ void close_round(BatchLat *lats, const uint32_t *active, const uint32_t n, BatchCounters *ctr,
+                                            uint32_t *chunk_lat, const uint32_t t, const uint32_t threads)
+{
+    for (uint32_t k = t; k < n; k += threads) {
+        BatchLat *L = lats + active[k];
+        if (!L->active)
+            continue;
+        L->sweeps_done += 1;
+        if (L->sweeps_left != kUnlimited)
+            L->sweeps_left -= 1;
+        if (chunk_lat && L->measure_every && L->sweeps_done % L->measure_every == 0) {
+            const uint32_t nch = (uint32_t)(((size_t)L->g.L0 * L->g.L1 + kChunkSites - 1) / kChunkSites);
+            const uint32_t base = atomicAdd(&ctr->measure_chunks, nch);
+            L->measure_base = base;
+            for (uint32_t c = 0; c < nch; ++c)
+                chunk_lat[base + c] = active[k];
+        }
+    }
+}
+
+struct CloseRound {  // what the merge of a round closes for its group (n 0: nothing)
+    const uint32_t *active;
+    uint32_t n;
+    BatchCounters *ctr;
+    uint32_t *chunk_lat;
+};
+
+// kWarps warps per item (merge_warps).  The last CTA closes the round for the group.
 template <uint32_t kWarps>
-__global__ void __launch_bounds__(kMergeThreads) kb_merge(const BatchLat *lats, const BlockRec *recs,
-                                                          const uint32_t total, unsigned int *fault)
+__global__ void __launch_bounds__(kMergeThreads) kb_merge(BatchLat *lats, const BlockRec *recs, const uint32_t total,
+                                                          unsigned int *fault, const CloseRound close)
 {
     __shared__ uint8_t list[kMergeThreads / 32][kMergeList];
     const uint32_t i = (blockIdx.x * kMergeThreads + threadIdx.x) / 32, item = i / kWarps;
     after_previous();
-    if (item < total) {
+    if (close.n && blockIdx.x + 1 == gridDim.x) {
+        close_round(lats, close.active, close.n, close.ctr, close.chunk_lat, threadIdx.x, kMergeThreads);
+    } else if (item < total) {
         const BlockRec r = recs[item];
-        const bool active = lats[r.lat].sweeps_left != 0;
+        const bool active = lats[r.lat].active != 0;
         merge_block<kWarps>(rec_geo(r), r.bxy & 0xFFFFu, r.bxy >> 16, i % kWarps, r.edge, r.labels, fault, r.linked,
                             list[threadIdx.x / 32], active);
     }
@@ -161,7 +198,7 @@ __global__ void __launch_bounds__(kMergeThreads) kb_resolve(const BatchLat *lats
     after_previous();
     if (item < total) {
         const BlockRec r = recs[item];
-        const bool active = lats[r.lat].sweeps_left != 0;
+        const bool active = lats[r.lat].active != 0;
         resolve_block<kWarps>(rec_geo(r), r.bxy & 0xFFFFu, r.bxy >> 16, i % kWarps, r.linked, r.labels, fault, active);
     }
 }
@@ -178,41 +215,21 @@ __global__ void __launch_bounds__(kFlipThreads, 6) kb_flip(const BatchLat *lats,
         // The budget is read beside the data, not ahead of it: a lattice whose budget ran out
         // leaves the lists at the engine's next call, so only the rest of the call in which it
         // finished reads (and does not write) its blocks.
-        const bool active = lats[r.lat].sweeps_left != 0;
+        const bool active = lats[r.lat].active != 0;
         flip_block<false, 4, kResolved>(rec_geo(r), r.bxy & 0xFFFFu, r.bxy >> 16, r.spins, r.labels, fault, smem, active);
         if (item + gridDim.x < total)
             __syncthreads();  // the next item reuses the shared memory
     }
 }
 
-// Closes a round after every phase kernel of it (before the measurement): each lattice that was
-// swept counts the sweep and spends one from its budget.  The kernels of the round read the
-// budget only to skip finished lattices, so it changes here, between rounds.
-// With chunk_lat (a round that measures), every lattice due for a sample (measure_every divides
-// its sweep count) appends its 4096-site chunks to the round's measure list, so kb_measure visits
-// only those.
-__global__ void kb_end_round(BatchLat *lats, const uint32_t *active, BatchCounters *ctr, uint32_t *chunk_lat)
+// close_round for every listed lattice, where no merge does it.
+__global__ void kb_end_round(BatchLat *lats, const uint32_t *active, BatchCounters *ctr)
 {
     after_previous();
-    const uint32_t n = ctr->n_active;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        BatchLat *L = lats + active[k];
-        if (L->sweeps_left != 0) {
-            L->sweeps_done += 1;
-            if (L->sweeps_left != kUnlimited)
-                L->sweeps_left -= 1;
-            if (chunk_lat && L->measure_every && L->sweeps_done % L->measure_every == 0) {
-                const uint32_t nch = (uint32_t)(((size_t)L->g.L0 * L->g.L1 + kChunkSites - 1) / kChunkSites);
-                const uint32_t base = atomicAdd(&ctr->measure_chunks, nch);
-                L->measure_base = base;
-                for (uint32_t c = 0; c < nch; ++c)
-                    chunk_lat[base + c] = active[k];
-            }
-        }
-    }
+    close_round(lats, active, ctr->n_active, ctr, nullptr, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// Energy / magnetisation of the lattices on this round's measure list (kb_end_round): CTAs pull
+// Energy / magnetisation of the lattices on this round's measure list (close_round): CTAs pull
 // 4096-site chunks from a device counter; per lattice int64 sums, the last chunk turns them into
 // FP64 accumulators.  A round whose list is empty costs one read per CTA.
 __global__ void __launch_bounds__(kMeasureThreads) kb_measure(BatchLat *lats, const uint32_t *chunk_lat,
@@ -347,6 +364,7 @@ struct swb_batch {
     uint32_t items_n = 0;           // block items in the list (the phase kernels' grid)
     uint64_t graph_version = ~0ull;  // lists_version the captured graphs were built for
     uint32_t grp_start[kRoundGroups] = {}, grp_count[kRoundGroups] = {};  // item ranges of the round's groups
+    uint32_t grp_lat[kRoundGroups] = {}, grp_lats[kRoundGroups] = {};     // their lattices in d_active
     cudaStream_t gstream[kRoundGroups] = {};
     cudaEvent_t fork = nullptr, join[kRoundGroups] = {};
     BatchCounters *d_ctr = nullptr;
@@ -375,7 +393,7 @@ struct swb_batch {
     bool lists_dirty = true;
     uint64_t round_count = 0;  // rounds queued so far (every listed lattice with budget left sweeps once)
     bool assign_all_shapes = true;  // an active lattice has a tile only the all-shapes assign compiles
-    int grid_measure = 0;
+    int grid_measure = 0, grid_round_measure = 0;  // full; for the listed lattices
     uint32_t smem_assign[2] = {}, smem_flip = 0;  // assign: one band, kBandsMax bands
     cudaGraphExec_t graph[2] = {nullptr, nullptr};   // [measure?]
     uint64_t series_cap = 1u << 16;
@@ -492,16 +510,21 @@ int rebuild_lists(swb_batch *b)
     }
     std::vector<uint2> items;
     items.reserve(bp[n]);
+    std::vector<uint32_t> by_group;  // d_active: the lattices, group by group
+    by_group.reserve(n);
     for (uint32_t q = 0; q < kRoundGroups; ++q) {
         b->grp_start[q] = (uint32_t)items.size();
+        b->grp_lat[q] = (uint32_t)by_group.size();
         for (uint32_t k = 0; k < n; ++k) {
             if (grp[k] != q)
                 continue;
             const Geo &g = b->lats[b->active[k]].d.g;
+            by_group.push_back(b->active[k]);
             for (uint32_t by = 0; by < g.nby; ++by)
                 for (uint32_t bx = 0; bx < g.nbx; ++bx)
                     items.push_back(make_uint2(b->active[k], by << 16 | bx));
         }
+        b->grp_lats[q] = (uint32_t)by_group.size() - b->grp_lat[q];
         b->grp_count[q] = (uint32_t)items.size() - b->grp_start[q];
     }
     if (items.size() > b->items_cap) {
@@ -535,6 +558,7 @@ int rebuild_lists(swb_batch *b)
         b->chunk_lat_cap = cap;
     }
     b->items_n = (uint32_t)items.size();
+    b->grid_round_measure = std::max(1, std::min<int>(b->grid_measure, (int)cp[n]));
     BatchCounters c{};
     c.n_active = n;
     c.total_chunks = cp[n];
@@ -544,7 +568,7 @@ int rebuild_lists(swb_batch *b)
         const std::vector<BlockRec> recs = make_recs(b, items);
         SWB_CUDA(cudaMemcpyAsync(b->d_recs, recs.data(), sizeof(BlockRec) * recs.size(), cudaMemcpyHostToDevice,
                                  b->stream));
-        SWB_CUDA(cudaMemcpyAsync(b->d_active, b->active.data(), n * 4, cudaMemcpyHostToDevice, b->stream));
+        SWB_CUDA(cudaMemcpyAsync(b->d_active, by_group.data(), n * 4, cudaMemcpyHostToDevice, b->stream));
     }
     SWB_CUDA(cudaMemcpyAsync(b->d_ctr, &c, sizeof(c), cudaMemcpyHostToDevice, b->stream));
     b->lists_dirty = false;
@@ -567,11 +591,12 @@ int launch_assign_b(swb_batch *b, const uint2 *items, uint32_t n, cudaStream_t s
     return launch_next(early, k, grid, threads, smem, st, b->d_lats, items, n, bands, ctr);
 }
 
-int launch_merge_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_t st, bool early)
+int launch_merge_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_t st, bool early, const CloseRound &close)
 {
     const uint32_t w = merge_warps(n);
     auto k = w == kEdgeParts ? kb_merge<kEdgeParts> : w == 1 ? kb_merge<1> : kb_merge<kMidWarps>;
-    return launch_next(early, k, merge_grid(n), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault);
+    return launch_next(early, k, merge_grid(n) + (close.n ? 1 : 0), kMergeThreads, 0, st, b->d_lats, recs, n, b->d_fault,
+                       close);
 }
 
 // kb_resolve, where the launch has one (few items: the flip chases the merged roots, as in swb_create).
@@ -592,27 +617,27 @@ int launch_flip_b(swb_batch *b, const BlockRec *recs, uint32_t n, cudaStream_t s
 
 // The phases of one sweep over a list of block items.
 int launch_phases_b(swb_batch *b, const uint2 *items, const BlockRec *recs, uint32_t n, cudaStream_t st,
-                    bool early = false, BatchCounters *ctr = nullptr, uint32_t full_items = kFullItems)
+                    bool early = false, BatchCounters *ctr = nullptr, const CloseRound &close = CloseRound{},
+                    uint32_t full_items = kFullItems)
 {
     if (int rc = launch_assign_b(b, items, n, st, early, ctr, full_items))
         return rc;
-    if (int rc = launch_merge_b(b, recs, n, st, early))
+    if (int rc = launch_merge_b(b, recs, n, st, early, close))
         return rc;
     if (int rc = launch_resolve_b(b, recs, n, st, early))
         return rc;
     return launch_flip_b(b, recs, n, st, early);
 }
 
-int launch_end_round(swb_batch *b, cudaStream_t st, bool measure, bool early = false)
+int launch_end_round(swb_batch *b, cudaStream_t st)
 {
-    return launch_next(early, kb_end_round, 4, 128, 0, st, b->d_lats, b->d_active, b->d_ctr,
-                       measure ? b->d_chunk_lat : nullptr);
+    return launch_next(false, kb_end_round, 4, 128, 0, st, b->d_lats, b->d_active, b->d_ctr);
 }
 
-// Kernels of one captured round: three or four phases per non-empty lattice group, end, measure.
+// Kernels of one round: three or four phases per non-empty lattice group, measure.
 uint32_t round_launches(const swb_batch *b, bool measure)
 {
-    uint32_t n = 1 + (measure ? 1 : 0);
+    uint32_t n = measure ? 1 : 0;
     for (uint32_t q = 0; q < kRoundGroups; ++q)
         n += b->grp_count[q] ? (b->grp_count[q] < kResolveItems ? 3 : 4) : 0;
     return n;
@@ -621,9 +646,12 @@ uint32_t round_launches(const swb_batch *b, bool measure)
 int launch_round(swb_batch *b, bool measure)
 {
     const bool alone = b->grp_count[1] == 0;  // one group: a single chain of kernels
+    auto close = [&](uint32_t q) {
+        return CloseRound{b->d_active + b->grp_lat[q], b->grp_lats[q], b->d_ctr, measure ? b->d_chunk_lat : nullptr};
+    };
     if (alone) {
         if (b->grp_count[0])
-            if (int rc = launch_phases_b(b, b->d_items, b->d_recs, b->grp_count[0], b->stream, true, b->d_ctr))
+            if (int rc = launch_phases_b(b, b->d_items, b->d_recs, b->grp_count[0], b->stream, true, b->d_ctr, close(0)))
                 return rc;
     } else {
         // The groups' sweeps run on their own streams: the end of one group's assign overlaps the
@@ -636,21 +664,23 @@ int launch_round(swb_batch *b, bool measure)
                 SWB_CUDA(cudaStreamCreateWithFlags(&b->gstream[q], cudaStreamNonBlocking));
             }
         }
+        // the previous round's measure list is emptied before either group closes its part of this one
+        static_assert(offsetof(BatchCounters, measure_chunks) == sizeof(unsigned int), "cleared with measure_next");
+        if (measure)
+            SWB_CUDA(cudaMemsetAsync(b->d_ctr, 0, 2 * sizeof(unsigned int), b->stream));
         SWB_CUDA(cudaEventRecord(b->fork, b->stream));
         for (uint32_t q = 0; q < kRoundGroups; ++q) {
             SWB_CUDA(cudaStreamWaitEvent(b->gstream[q], b->fork, 0));
             if (int rc = launch_phases_b(b, b->d_items + b->grp_start[q], b->d_recs + b->grp_start[q], b->grp_count[q],
-                                         b->gstream[q], false, q == 0 ? b->d_ctr : nullptr))
+                                         b->gstream[q], false, nullptr, close(q)))
                 return rc;
             SWB_CUDA(cudaEventRecord(b->join[q], b->gstream[q]));
             SWB_CUDA(cudaStreamWaitEvent(b->stream, b->join[q], 0));
         }
     }
-    if (int rc = launch_end_round(b, b->stream, measure, alone))
-        return rc;
     if (measure)
-        return launch_next(alone, kb_measure, b->grid_measure, kMeasureThreads, 0, b->stream, b->d_lats, b->d_chunk_lat,
-                           b->d_ctr);
+        return launch_next(alone, kb_measure, b->grid_round_measure, kMeasureThreads, 0, b->stream, b->d_lats,
+                           b->d_chunk_lat, b->d_ctr);
     return SWB_OK;
 }
 
@@ -1114,7 +1144,7 @@ int swb_batch_sweep_timed(swb_batch *b, uint32_t n_rounds, int per_kernel, float
             if ((rc = launch_assign_b(b, b->d_items, b->items_n, b->stream, false, nullptr, kFullItems)))
                 break;
             SWB_CUDA(cudaEventRecord(ev[2], b->stream));
-            if ((rc = launch_merge_b(b, b->d_recs, b->items_n, b->stream, false)))
+            if ((rc = launch_merge_b(b, b->d_recs, b->items_n, b->stream, false, CloseRound{})))
                 break;
             SWB_CUDA(cudaEventRecord(ev[3], b->stream));
             // resolve + flip: the reference's ResolveLabels and FlipClusters
@@ -1123,7 +1153,7 @@ int swb_batch_sweep_timed(swb_batch *b, uint32_t n_rounds, int per_kernel, float
             if ((rc = launch_flip_b(b, b->d_recs, b->items_n, b->stream, false)))
                 break;
             SWB_CUDA(cudaEventRecord(ev[4], b->stream));
-            if ((rc = launch_end_round(b, b->stream, false)))
+            if ((rc = launch_end_round(b, b->stream)))
                 break;
             b->round_count += 1;
             SWB_CUDA(cudaEventSynchronize(ev[4]));
@@ -1412,7 +1442,7 @@ int update_host_rounds(swb_batch *b, uint32_t count, const uint32_t *ids, const 
             uint8_t *const *dst = (r & 1) ? const_cast<uint8_t *const *>(spins_in) : spins_out;
             if (gi[1])
                 if (int rc = launch_phases_b(b, b->d_io_items, b->d_io_recs, (uint32_t)gi[1], b->stream, false, nullptr,
-                                             kIoFullItems))
+                                             CloseRound{}, kIoFullItems))
                     return rc;
             for (uint32_t g = 0; g < G; ++g) {
                 if (r)  // the previous round's copies out of this group have landed
@@ -1435,12 +1465,13 @@ int update_host_rounds(swb_batch *b, uint32_t count, const uint32_t *ids, const 
                 kb_stage_copy<<<sgrid, 256, 0, b->stream>>>(b->d_copies + gs[g], b->d_stage, 1);
                 SWB_LAUNCHED();
                 if (int rc = launch_phases_b(b, b->d_io_items + gi[g + 1], b->d_io_recs + gi[g + 1],
-                                             (uint32_t)(gi[g + 2] - gi[g + 1]), b->stream, false, nullptr, kIoFullItems))
+                                             (uint32_t)(gi[g + 2] - gi[g + 1]), b->stream, false, nullptr, CloseRound{},
+                                             kIoFullItems))
                     return rc;
                 kb_stage_copy<<<sgrid, 256, 0, b->stream>>>(b->d_copies + gs[g], b->d_stage, 0);
                 SWB_LAUNCHED();
                 if (g + 1 == G) {  // every listed and unlisted lattice has swept: close the round
-                    if (int rc = launch_end_round(b, b->stream, false))
+                    if (int rc = launch_end_round(b, b->stream))
                         return rc;
                     b->round_count += 1;
                 }
