@@ -32,13 +32,17 @@ constexpr uint32_t kMeasureThreads = 256;      // measure: one thread per 16 sit
 constexpr uint32_t kFlipThreads = 256;         // flip: four quads of a 128 x 32 block per thread
 constexpr uint32_t kChunkSites = 4096;         // measure work item
 constexpr uint32_t kRoundGroups = 2;           // lattice groups whose sweeps run side by side in a round
-constexpr uint32_t kFullItems = 592;           // launches of fewer block items run the assign in bands
+// Launches of fewer block items run the assign in bands: 166 items 24.7 us a round with 4 bands and 27.4
+// with one, 416 items 32.3 and 33.7; 440 items 32.1 and 31.1, 1515 items 71 and 57.
+constexpr uint32_t kFullItems = 430;
 // The same beside host copies: a group's sweep sits between its copies, so its latency counts for more
 // than its throughput (512-lattice mix through host buffers, 8 groups of about 1300 items: 0.98 ms a
 // round in bands, 1.13 with one band).
 constexpr uint32_t kIoFullItems = 4096;
 constexpr uint32_t kResolveItems = 1024;       // launches of fewer items have no kb_resolve
-constexpr uint32_t kTwoGroupItems = 1184;      // rounds of fewer items run as one group
+// Rounds of fewer items run as one group, launched directly and early: 1916 items 65 us a round against
+// 70 in two groups as a graph; 2696 items 81 against 78, 5156 items 148 against 136.
+constexpr uint32_t kTwoGroupItems = 2304;
 constexpr uint32_t kUnlimited = 0xFFFFFFFFu;   // sweeps_left value that never runs out
 
 struct BatchLat {

@@ -76,3 +76,26 @@ def test_batched_strips_bit_exact_vs_oracle(gpu, oracle, W, block):
             assert np.array_equal(b.get_spins(i), spins)
             st, a, c, it = b.get_rng(i)
             assert np.array_equal(st, rng.state) and np.array_equal(it, rng.iteration) and np.array_equal(a, rng.a)
+
+
+@pytest.mark.parametrize("L1", [2016, 2048])
+def test_batched_rounds_in_one_and_two_groups(gpu, oracle, L1):
+    """2290 and 2338 block items, either side of the line between rounds launched directly as one group and
+    rounds of two groups side by side; budgets that end in different rounds."""
+    shapes = [(2048, 2048, 5), (2048, L1, 3), (1024, 1024, 4), (96, 64, 2)]
+    if L1 == 2048:
+        shapes.append((512, 256, 5))
+    with gpu.BatchedSW(capacity=8) as b:
+        ids = []
+        for k, (L0, M, sweeps) in enumerate(shapes):
+            ids.append(b.add(L0, M, 2.2691853, k + 1, (16, 8)))
+            b.hot_start(ids[-1], k + 1)
+            b.set_schedule(ids[-1], sweeps, 2)
+        b.sweep(6, measure=True)
+        for k, (i, (L0, M, sweeps)) in enumerate(zip(ids, shapes)):
+            with gpu.SwendsenWang2D(L0, M, (16, 8), 16, k + 1) as sw:
+                sw.hot_start(k + 1)
+                sw.update(2.2691853, sweeps, 2)
+                assert b.status(i) == (0, sweeps)
+                assert np.array_equal(b.get_spins(i), sw.get_spins())
+                assert np.array_equal(b.samples(i), sw.samples())
