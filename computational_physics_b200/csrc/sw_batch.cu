@@ -117,10 +117,11 @@ __device__ __forceinline__ Geo rec_geo(const BlockRec &r)
 // Budgets change between a round's merge and the next round's assign (close_round), so the draws and the
 // choice of the lattices to sweep may run beside the previous round's last kernel.  With ctr (the first
 // assign of a round) the measure list of the previous round is emptied.
-template <int W, bool kAllShapes>
-__global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) kb_assign(BatchLat *lats, const uint2 *items,
-                                                                          const uint32_t total, const uint32_t bands,
-                                                                          BatchCounters *ctr)
+// kOneBand: items of one band; 9 CTAs an SM leave room for 56 registers and, beside the other group, for its
+// merge and flip (512-lattice mix round 243 us; 252 with 10 or 12 CTAs, 251 with 8).
+template <int W, bool kAllShapes, bool kOneBand>
+__global__ void __launch_bounds__(kOneBand ? kStripThreads : kStripThreads * kBandsMax, kOneBand ? 9 : 3)
+    kb_assign(BatchLat *lats, const uint2 *items, const uint32_t total, const uint32_t bands, BatchCounters *ctr)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const uint2 d = load_item(items, blockIdx.x, total);
@@ -128,9 +129,9 @@ __global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) kb_assign(BatchL
     const bool on = blockIdx.x < total && L->sweeps_left != 0;
     if (on) {
         const Geo g = L->g;
-        assign_strips_any<W, false, false, true, kAllShapes>(g, d.y & 0xFFFFu, d.y >> 16, bands, L->spins, L->labels,
-                                                             L->rng_state, L->rng_sel, L->rng_iter, L->thr, L->edge,
-                                                             AssignDump{}, MeasureArgs{}, smem);
+        assign_strips_any<W, false, false, true, kAllShapes>(g, d.y & 0xFFFFu, d.y >> 16, kOneBand ? 1u : bands,
+                                                             L->spins, L->labels, L->rng_state, L->rng_sel, L->rng_iter,
+                                                             L->thr, L->edge, AssignDump{}, MeasureArgs{}, smem);
     } else {
         after_previous();
     }
@@ -580,6 +581,14 @@ int rebuild_lists(swb_batch *b)
     return SWB_OK;
 }
 
+template <bool kOneBand>
+auto assign_kernel(const swb_batch *b)
+{
+    return b->W == 8    ? kb_assign<8, true, kOneBand>
+           : b->W == 32 ? kb_assign<32, true, kOneBand>
+                        : b->assign_all_shapes ? kb_assign<16, true, kOneBand> : kb_assign<16, false, kOneBand>;
+}
+
 // One CTA per block item (at least one CTA): the hardware scheduler interleaves the phases of
 // co-resident CTAs better than a persistent loop does.  `items` / `n` is any list of block
 // items: the whole round's, or one group of update_host's pipeline.
@@ -590,8 +599,7 @@ int launch_assign_b(swb_batch *b, const uint2 *items, uint32_t n, cudaStream_t s
 {
     const uint32_t grid = std::max(n, 1u), bands = n >= full_items ? 1 : kBandsMax;
     const uint32_t threads = kStripThreads * bands, smem = b->smem_assign[bands != 1];
-    auto k = b->W == 8 ? kb_assign<8, true> : b->W == 32 ? kb_assign<32, true>
-                                            : b->assign_all_shapes ? kb_assign<16, true> : kb_assign<16, false>;
+    auto k = bands == 1 ? assign_kernel<true>(b) : assign_kernel<false>(b);
     return launch_next(early, k, grid, threads, smem, st, b->d_lats, items, n, bands, ctr);
 }
 

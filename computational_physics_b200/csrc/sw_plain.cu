@@ -77,18 +77,18 @@ inline uint32_t assign_bands(const Geo &g) { return g.nbx * g.nby >= kFullBlocks
 // shape (TYc 0: any height).  `dump` is all null in a plain sweep; swb_sweep_dumped runs the same
 // instance with dumps on.  kMeasure: the instance that also measures the spins it starts from
 // (`meas`), used by the sweep after a measured one; a separate instance so the others carry none
-// of its registers.
-template <int W, int TXc, int TYc, bool kMeasure>
-__global__ void __launch_bounds__(kStripThreads * kBandsMax, 3) k_assign(const Geo g, const uint8_t *spins,
-                                                              uint32_t *labels,
-                                                              uint32_t *__restrict__ rng_state,
-                                                              uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter,
-                                                              const uint32_t thr, uint32_t *edge,
-                                                              const AssignDump dump, const MeasureArgs meas, const uint32_t bands)
+// of its registers.  kOneBand: blocks of one band, which drops the bands' arithmetic and leaves room for
+// 48 registers a thread (16384^2 at T_c: 868 us a launch; 885 with 40 registers and 12 CTAs an SM, 903 with
+// 56 and 9; 903 when the same instance served several bands).
+template <int W, int TXc, int TYc, bool kMeasure, bool kOneBand>
+__global__ void __launch_bounds__(kOneBand ? kStripThreads : kStripThreads * kBandsMax, kOneBand ? 10 : 3)
+    k_assign(const Geo g, const uint8_t *spins, uint32_t *labels, uint32_t *__restrict__ rng_state,
+             uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter, const uint32_t thr, uint32_t *edge,
+             const AssignDump dump, const MeasureArgs meas, const uint32_t bands)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    assign_strips<W, TXc, TYc, kMeasure, true, true>(g, blockIdx.x, blockIdx.y, bands, spins, labels, rng_state, rng_sel,
-                                               rng_iter, thr, edge, dump, meas, smem);
+    assign_strips<W, TXc, TYc, kMeasure, true, true>(g, blockIdx.x, blockIdx.y, kOneBand ? 1u : bands, spins, labels,
+                                                     rng_state, rng_sel, rng_iter, thr, edge, dump, meas, smem);
 }
 
 // The assign phase of swb_sweep_recorded, labelling tile by tile.
@@ -258,9 +258,10 @@ int launch_assign_k(swb_lattice *h, float p_add, const AssignDump &dump, const M
     const Geo &g = h->g;
     const dim3 grid(g.nbx, g.nby), block((g.BX + 31) / 32 * 32 * h->bands);
     const uint32_t thr = accept_threshold(p_add);
-    auto k = meas.obs ? k_assign<W, TXc, TYc, true> : k_assign<W, TXc, TYc, false>;
-    return launch_next(early_launch(h), k, grid, block, h->smem_assign, h->stream, g, h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, thr,
-                       h->edge, dump, meas, h->bands);
+    auto k = h->bands == 1 ? (meas.obs ? k_assign<W, TXc, TYc, true, true> : k_assign<W, TXc, TYc, false, true>)
+                           : (meas.obs ? k_assign<W, TXc, TYc, true, false> : k_assign<W, TXc, TYc, false, false>);
+    return launch_next(early_launch(h), k, grid, block, h->smem_assign, h->stream, g, h->spins, h->labels, h->rng_state,
+                       h->rng_sel, h->rng_iter, thr, h->edge, dump, meas, h->bands);
 }
 
 // The instance a plain sweep of this handle runs (compile-time tile shape for the common
