@@ -32,12 +32,12 @@ constexpr uint32_t kMeasureThreads = 256;      // measure: one thread per 16 sit
 constexpr uint32_t kFlipThreads = 256;         // flip: four quads of a 128 x 32 block per thread
 constexpr uint32_t kChunkSites = 4096;         // measure work item
 constexpr uint32_t kRoundGroups = 2;           // lattice groups whose sweeps run side by side in a round
-// Launches of fewer block items run the assign in bands: 166 items 24.7 us a round with 4 bands and 27.4
-// with one, 416 items 32.3 and 33.7; 440 items 32.1 and 31.1, 1515 items 71 and 57.
-constexpr uint32_t kFullItems = 430;
+// Launches of fewer block items run the assign in bands: 166 items 24.6 us a round with 4 bands and 27.1
+// with one, 383 items 31.4 and 32.0; 416 items 32.4 and 31.6, 440 items 32.1 and 30.4.
+constexpr uint32_t kFullItems = 400;
 // The same beside host copies: a group's sweep sits between its copies, so its latency counts for more
 // than its throughput (512-lattice mix through host buffers, 8 groups of about 1300 items: 0.98 ms a
-// round in bands, 1.13 with one band).
+// round in bands, 1.15 with one band).
 constexpr uint32_t kIoFullItems = 4096;
 constexpr uint32_t kResolveItems = 1024;       // launches of fewer items have no kb_resolve
 // Rounds of fewer items run as one group, launched directly and early: 1916 items 65 us a round against
