@@ -1,8 +1,8 @@
 // Swendsen-Wang sweep for the 2D Ising model on one B200 (sm_100a), behind the C ABI of
 // include/swb200.h.
 //
-// One sweep = four kernels on the handle's stream (reference phases in brackets,
-// ising/src/swendsen_wang.cpp:94-112):
+// One sweep = four kernels on the handle's stream, or one for small lattices (sw_whole.cuh); reference
+// phases in brackets (ising/src/swendsen_wang.cpp:94-112):
 //
 //   k_assign  [AssignLabels + the in-block part of MergeLabels]  one CTA per block of
 //             TBX x TBY tiles, one warp per 32-column strip (sw_strip.cuh): lcg32 draws, bond
@@ -68,9 +68,10 @@ int fail(int code, const char *fmt, ...)
 
 constexpr uint32_t kTilesThreads = 512;  // CTA of the recorded sweep's assign
 
-// Bands of an assign block: one where the lattice's blocks fill the GPU with a warp per strip, else
-// a band per tile row (up to kBandsMax).
-constexpr uint32_t kFullBlocks = 592;
+// Bands of an assign block: a band per tile row (up to kBandsMax) as long as all blocks are resident at once
+// (3 CTAs of 16 warps on each of 148 SMs), else one, a warp per strip.  us a sweep, bands / one band: 256 blocks
+// (1024^2) 27.3 / 29.4, 320 27.4 / 27.2, 420 34.2 / 39.1, 430 28.6 / 30.4; 480 39.9 / 34.8, 512 37.4 / 30.7, 1024 47.1 / 38.9.
+constexpr uint32_t kFullBlocks = 3 * 148 + 1;
 inline uint32_t assign_bands(const Geo &g) { return g.nbx * g.nby >= kFullBlocks ? 1 : std::min(g.TBY, kBandsMax); }
 
 // The assign phase of a plain sweep (assign_strips): one warp per 32-column strip.  TXc, TYc: the tile

@@ -1,6 +1,6 @@
 """The assign phase's strips and bands (csrc/sw_strip.cuh) where they can go wrong: partial strips, extents
 that allow only 4- or 2-byte loads, tile heights that leave a short band or a partial tile row, every tile
-width with every lcg width (one to four passes of draws per tile row), one band (at least 592 blocks) and
+width with every lcg width (one to four passes of draws per tile row), one band (at least 445 blocks) and
 several, and more unions in a strip than its list holds.  Bonds, block labels, resolved labels, spins
 and lcg32 streams bit for bit against the restatement."""
 import numpy as np
