@@ -79,10 +79,11 @@ inline uint32_t assign_bands(const Geo &g) { return g.nbx * g.nby >= kFullBlocks
 // instance with dumps on.  kMeasure: the instance that also measures the spins it starts from
 // (`meas`), used by the sweep after a measured one; a separate instance so the others carry none
 // of its registers.  kOneBand: blocks of one band, which drops the bands' arithmetic and leaves room for
-// 48 registers a thread (16384^2 at T_c: 868 us a launch; 885 with 40 registers and 12 CTAs an SM, 903 with
-// 56 and 9; 903 when the same instance served several bands).
+// 56 registers a thread, 9 CTAs an SM.  us a sweep at T_c, one lattice / three at a time on their own streams: 16384^2
+// 1365 / 1311 (10 CTAs of 48 registers 1331 / 1440, 8 of 64 1405 / 1352, 12 of 40 1347 / 1455), 4096^2 117 / 88 (112 / 95,
+// 118 / 89, 114 / 95): 10 are faster for a lattice alone, but lose more beside others.
 template <int W, int TXc, int TYc, bool kMeasure, bool kOneBand>
-__global__ void __launch_bounds__(kOneBand ? kStripThreads : kStripThreads * kBandsMax, kOneBand ? 10 : 3)
+__global__ void __launch_bounds__(kOneBand ? kStripThreads : kStripThreads * kBandsMax, kOneBand ? 9 : 3)
     k_assign(const Geo g, const uint8_t *spins, uint32_t *labels, uint32_t *__restrict__ rng_state,
              uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter, const uint32_t thr, uint32_t *edge,
              const AssignDump dump, const MeasureArgs meas, const uint32_t bands)

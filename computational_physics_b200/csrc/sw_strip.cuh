@@ -18,7 +18,7 @@
 // With many blocks a block is one band (4 warps: no seams between bands, and instruction issue is what
 // bounds it: 2.5 warp instructions per site, of which scan 0.8, draws 0.7, unions 0.5, labels 0.3, the
 // rest 0.2); with few, a band per tile row (up to 16 warps), which shortens every warp's serial walk.
-// 16384^2 with 16 x 8 tiles: 868 us a launch (1305 with staged spins, bond words through shared memory and
+// 16384^2 with 16 x 8 tiles: 903 us a launch (1305 with staged spins, bond words through shared memory and
 // a find per site).
 #pragma once
 
