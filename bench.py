@@ -258,11 +258,11 @@ def assign_bytes(n_sites: int, n_tiles: int, W: int) -> float:
 # DRAM traffic of one assign pass over a workload (dram__bytes_read.sum + dram__bytes_write.sum)
 # from one ncu capture of the same kernel, per site: the batched mix of 512 lattices (39,603,200
 # sites; the round runs its two lattice groups as two launches: 33,091,072 + 33,103,872 B read,
-# 35,633,408 + 35,014,400 B written) and one 8192 x 8192 lattice, tile 16 x 8 (111,611,392 B read
-# + 253,764,608 B written).  Traffic grows with the sites swept, so other sizes scale by their
+# 35,633,408 + 35,014,400 B written) and one 8192 x 8192 lattice, tile 16 x 8 (111,595,520 B read
+# + 253,265,152 B written).  Traffic grows with the sites swept, so other sizes scale by their
 # site count.
 ASSIGN_TRAFFIC_PER_SITE = {"kb_assign": (33_091_072 + 33_103_872 + 35_633_408 + 35_014_400) / 39_603_200,
-                           "k_assign": (111_611_392 + 253_764_608) / 8192 ** 2}
+                           "k_assign": (111_595_520 + 253_265_152) / 8192 ** 2}
 
 
 def flip_bytes(n_sites: int) -> float:
