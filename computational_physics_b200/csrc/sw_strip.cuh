@@ -52,7 +52,7 @@ __host__ __device__ inline StripSmem strip_smem(const Geo &g, uint32_t W, uint32
     s.last = s.words + ns * g.BY * 16;                 // [band][strip] {y, x} bonds of the piece's last row
     s.draws = s.last + ns * bands * 8;                 // [band][strip][dcap]
     s.sums = s.draws + ns * bands * s.dcap * 4;        // energy and magnetisation sums, deep flag, edge words 0, 5, 6
-    s.pairs = s.sums + 32;                             // the five (a, c) pairs of lcg32
+    s.pairs = (s.sums + 32 + 7) & ~7u;                 // the five (a, c) pairs of lcg32, 8 bytes each
     s.total = s.pairs + 40;
     return s;
 }

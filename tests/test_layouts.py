@@ -49,3 +49,52 @@ def test_3d_assign_layout(tmp_path):
     assert len(rows) == 3 * 3 * 8 * 8
     assert [r[:4] for r in rows if r[4]] == []  # (W, tile) with an area off its alignment
     assert [r[:4] for r in rows if r[5]] == []  # (W, tile) that does not fit
+
+
+STRIPS = r"""
+#include "sw_strip.cuh"
+#include "sw_whole.cuh"
+#include <cstdio>
+using namespace swb;
+int main()
+{
+    for (uint32_t W = 8; W <= 32; W *= 2) {
+        const uint32_t most[2] = {strip_smem_max(W, 1), strip_smem_max(W, kBandsMax)};
+        for (uint32_t tx = 8; tx <= 32; tx *= 2)
+            for (uint32_t ty = 2; ty <= 32; ++ty) {
+                uint32_t misaligned = 0, large = 0;
+                for (uint32_t tbx = 1; tbx <= 128 / tx; ++tbx)
+                    for (uint32_t tby = 1; tby == 1 || tby * ty <= 32; ++tby)
+                        for (uint32_t bands = 1; bands <= kBandsMax; ++bands) {
+                            const Geo g = make_geo(1024, 1024, tx, ty, tbx, tby);
+                            const StripSmem s = strip_smem(g, W, bands);
+                            // parent and words: uint4; last and pairs: uint2; draws, sums: 32 bits
+                            misaligned += s.parent % 16 || s.words % 16 || s.last % 8 || s.draws % 4 || s.sums % 4 ||
+                                          s.pairs % 8;
+                            large += s.total > 48 * 1024 || (bands == 1 && s.total > most[0]) ||
+                                     (bands == kBandsMax && s.total > most[1]);
+                        }
+                // the one-kernel form, where make_whole takes the lattice
+                for (uint32_t L0 = 2; L0 <= 1056; L0 += L0 < 130 ? 2 : 62)
+                    for (uint32_t L1 = 2; L1 <= 1056; L1 += L1 < 130 ? 2 : 62) {
+                        const Whole w = make_whole(L0, L1, tx, ty);
+                        if (!w.ctas)
+                            continue;
+                        const WholeSmem s = whole_smem(w, W);
+                        // parent and scan: uint4; raw and pairs: uint2; the rest 32 bits
+                        misaligned += w.pitch % 4 || s.raw % 8 || s.scan % 16 || s.pairs % 8 ||
+                                      (s.spin | s.work | s.counts | s.edge | s.sums) % 4;
+                        large += s.total > kWholeSmemMax;
+                    }
+                std::printf("%u %u %u %u %u\n", W, tx, ty, misaligned, large);
+            }
+    }
+}
+"""
+
+
+def test_2d_assign_layouts(tmp_path):
+    rows = [tuple(map(int, line.split())) for line in _run(tmp_path, STRIPS)]
+    assert len(rows) == 3 * 3 * 31
+    assert [r[:3] for r in rows if r[3]] == []  # (W, tile) with an area off its alignment
+    assert [r[:3] for r in rows if r[4]] == []  # (W, tile) that does not fit
