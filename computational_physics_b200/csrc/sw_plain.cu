@@ -253,6 +253,10 @@ int set_device(const swb_lattice *h)
 }
 
 bool early_launch(const swb_lattice *h) { return h->g.nbx * h->g.nby < kEarlyBlocks; }
+// The assign draws before it waits for its predecessor, so that one must not write the streams.  No phase
+// kernel that comes before an assign does, but k_whole does: where plain sweeps run it, a dumped or timed
+// sweep's assign may follow it directly and is launched the ordinary way.
+bool early_assign(const swb_lattice *h) { return early_launch(h) && !h->whole.ctas; }
 
 template <int W, int TXc, int TYc>
 int launch_assign_k(swb_lattice *h, float p_add, const AssignDump &dump, const MeasureArgs &meas)
@@ -262,7 +266,7 @@ int launch_assign_k(swb_lattice *h, float p_add, const AssignDump &dump, const M
     const uint32_t thr = accept_threshold(p_add);
     auto k = h->bands == 1 ? (meas.obs ? k_assign<W, TXc, TYc, true, true> : k_assign<W, TXc, TYc, false, true>)
                            : (meas.obs ? k_assign<W, TXc, TYc, true, false> : k_assign<W, TXc, TYc, false, false>);
-    return launch_next(early_launch(h), k, grid, block, h->smem_assign, h->stream, g, h->spins, h->labels, h->rng_state,
+    return launch_next(early_assign(h), k, grid, block, h->smem_assign, h->stream, g, h->spins, h->labels, h->rng_state,
                        h->rng_sel, h->rng_iter, thr, h->edge, dump, meas, h->bands);
 }
 

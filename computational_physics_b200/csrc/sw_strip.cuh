@@ -282,8 +282,9 @@ __device__ __forceinline__ void strip_accept(const Geo &g, const uint32_t *d, co
 // Block (bxi, byi) of a lattice by a CTA of 32 threads per strip and band; smem holds
 // strip_smem(g, W, bands).total bytes.  kMeasure: also add the block's energy and magnetisation sums
 // (of the spins the sweep starts from) to meas.obs.  kMayDump: `dump` may ask for the bonds and the
-// block's labels.  kEarly: the kernel was launched by launch_next; the draws, which need nothing of
-// the previous kernels (the streams were last written a sweep ago), come before the wait for them.
+// block's labels.  kEarly: the kernel was launched by launch_next; the draws come before the wait
+// for the previous kernel, which must not write the streams (the previous sweep's assign, which does, is two
+// or more kernels back).
 template <int W, int TXc, int TYc, bool kMeasure, bool kMayDump, bool kEarly>
 __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, const uint32_t byi,
                                               const uint32_t bands, const uint8_t *spins,
