@@ -152,7 +152,10 @@ __device__ __forceinline__ void strip_draws(const Geo &g, const uint32_t bxi, co
         const uint32_t onm = __ballot_sync(0xffffffffu, on);
         if (onm == 0)
             continue;
-        uint32_t st = t.st, sel = t.sel, it = t.it;
+        // swb_sweep_static's indices are its caller's: one past the last pair acts as the last, as in lcg_param_a,
+        // and reads nothing behind the table of pairs.  (Not where they are loaded, which would wait for the
+        // load a pass early: 16384^2 sweep 1.32 -> 1.36 ms.)
+        uint32_t st = t.st, sel = min(t.sel, 4u), it = t.it;
         uint2 ac = pairs[sel];
         // The parameter rotation of LCG32_State::Update (random/src/lcg32.cpp:51-84): before
         // update itn when itn is a multiple of 15, the (a, c) pairs rotate by
