@@ -252,7 +252,9 @@ int set_device(const swb_lattice *h)
     return SWB_OK;
 }
 
-bool early_launch(const swb_lattice *h) { return h->g.nbx * h->g.nby < kEarlyBlocks; }
+// kEarlyBlocks, of 128 columns: narrower blocks count by their strips, the assign's warps (2048 blocks of 32 x 32
+// are a quarter of that work: 32 x 65536 at T_c 48.6 us a sweep the ordinary way, 40.4 early).
+bool early_launch(const swb_lattice *h) { return h->g.nbx * h->g.nby * ((h->g.BX + 31) / 32) < 4 * kEarlyBlocks; }
 // The assign draws before it waits for its predecessor, so that one must not write the streams.  No phase
 // kernel that comes before an assign does, but k_whole does: where plain sweeps run it, a dumped or timed
 // sweep's assign may follow it directly and is launched the ordinary way.

@@ -48,3 +48,24 @@ def test_label_rows_in_a_batch(gpu, oracle, block, many):
             for _ in range(2):
                 oracle.sweep(spins, *tile, rng, T=T)
             assert np.array_equal(b.get_spins(i), spins)
+
+
+@pytest.mark.parametrize("L0,L1,tile,W", [(2, 65600, (16, 8), 16), (30, 66000, (8, 8), 8), (64, 66000, (32, 16), 32)])
+def test_narrow_lattices_of_many_blocks(gpu, oracle, L0, L1, tile, W):
+    """More than 2048 blocks of one or two strips: sweeps and samples one after the other."""
+    spins = oracle.hot_start(L0, L1, 4)
+    rng = oracle.rng_init(W, num_tiles(L0, L1, *tile), 6)
+    want = []
+    with gpu.SwendsenWang2D(L0, L1, tile, W, 6) as sw:
+        geo = sw.geometry()
+        assert geo["blocks_x"] * geo["blocks_y"] > 2048
+        sw.set_spins(spins)
+        sw.update(T, 4, measure_every=2)
+        for k in range(4):
+            oracle.sweep(spins, *tile, rng, T=T)
+            if k % 2:
+                want.append(oracle.energy_magnetization(spins))
+        assert [tuple(s) for s in sw.samples()] == want
+        assert np.array_equal(sw.get_spins(), spins)
+        st, a, c, it = sw.get_rng()
+        assert np.array_equal(st, rng.state) and np.array_equal(it, rng.iteration)
