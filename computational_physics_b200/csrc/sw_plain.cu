@@ -66,7 +66,9 @@ int fail(int code, const char *fmt, ...)
     return code;
 }
 
-constexpr uint32_t kTilesThreads = 512;  // CTA of the recorded sweep's assign
+// CTA of the recorded sweep's assign, at most: a block's lcg lanes (8 x 8 tiles with W 16 have 1024; in two passes
+// of 512 a recorded 512^2 sweep took 580 us, now 522).
+constexpr uint32_t kTilesThreads = 1024;
 
 // Bands of an assign block: a band per tile row (up to kBandsMax) as long as all blocks are resident at once
 // (3 CTAs of 16 warps on each of 148 SMs), else one, a warp per strip.  us a sweep, bands / one band: 256 blocks
