@@ -56,17 +56,18 @@ __device__ __forceinline__ uint32_t label_global3(const Geo3 &g, uint32_t bxi, u
 // The draws of one sweep for a piece (tile rows [ty0, ty0 + nty) of tile layer tz, every tile column of
 // the block), as strip_draws: tile q (tile rows outer, columns inner) is segment q % (32 / W) of pass
 // q / (32 / W); update u of pass p leaves its ballot in d[p * total + u].  A tile that lacks a row idles
-// through it.
+// through it.  This warp takes the passes first, first + step, ...
 template <int W, int TX>
 __device__ __forceinline__ void draws_piece3(const Geo3 &g, const uint32_t bxi, const uint32_t ty_first,
                                              const uint32_t nty, const uint32_t tz, uint32_t *d, const Draws3 &D,
-                                             const uint2 *pairs, uint32_t *__restrict__ rng_state,
-                                             uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter,
-                                             const uint32_t thr)
+                                             const uint32_t first, const uint32_t step, const uint2 *pairs,
+                                             uint32_t *__restrict__ rng_state, uint8_t *__restrict__ rng_sel,
+                                             uint32_t *__restrict__ rng_iter, const uint32_t thr)
 {
     constexpr uint32_t kTps = 32 / TX, kPer = 32 / W;
     const uint32_t TY = g.TY, TZ = g.TZ, lane32 = threadIdx.x & 31, lane = lane32 % W;
-    for (uint32_t p = 0; p * kPer < nty * kTps; ++p, d += D.total) {
+    d += first * D.total;
+    for (uint32_t p = first; p * kPer < nty * kTps; p += step, d += step * D.total) {
         const uint32_t q = p * kPer + lane32 / W, tcol = q % kTps;
         const uint32_t tgx = bxi * g.TBX + tcol, tgy = ty_first + q / kTps;
         const bool on = q < nty * kTps && tcol < g.TBX && tgx < g.n0 && tgy < g.n1;
@@ -238,14 +239,16 @@ k3_assign(const Geo3 g, const uint8_t *spins, uint32_t *labels, uint32_t *__rest
     const uint32_t x0 = bxi * g.BX, y0 = byi * g.BY, z0 = bzi * g.BZ;
     const uint32_t bxv = min(g.BX, g.L0 - x0), byv = min(g.BY, g.L1 - y0), bzv = min(g.BZ, g.L2 - z0);
     const size_t plane = (size_t)g.L0 * g.L1;
-    // the piece: rows [yp, yp + nj) of layers [zp, zp + nk) of the block (np rows to a full layer)
-    const uint32_t tz = warp / g.pcy, typ = (warp - tz * g.pcy) * g.py;
+    // the piece: rows [yp, yp + nj) of layers [zp, zp + nk) of the block.  `share` warps take its draws
+    // between them (draw_share3), the first of them all the rest.
+    const uint32_t np = pieces3(g), share = nwarps / np, piece = share == 1 ? warp : warp % np;
+    const uint32_t tz = piece / g.pcy, typ = (piece - tz * g.pcy) * g.py;
     const uint32_t yp = typ * g.TY, zp = tz * g.TZ, PY = g.py * g.TY;
-    const bool here = warp < pieces3(g) && yp < byv && zp < bzv;
+    const bool exists = yp < byv && zp < bzv, here = exists && warp < np;
     const uint32_t nj = here ? min(PY, byv - yp) : 0, nk = here ? min(g.TZ, bzv - zp) : 0;
-    uint32_t *work = reinterpret_cast<uint32_t *>(smem + S.work) + warp * S.wcap;
-    uint16_t *links = reinterpret_cast<uint16_t *>(smem + S.links) + warp * k3Links;
-    uint4 *scan = reinterpret_cast<uint4 *>(smem + S.scan) + warp * S.rows * 2;
+    uint32_t *work = reinterpret_cast<uint32_t *>(smem + S.work) + piece * S.wcap;
+    uint16_t *links = reinterpret_cast<uint16_t *>(smem + S.links) + piece * k3Links;
+    uint4 *scan = reinterpret_cast<uint4 *>(smem + S.scan) + piece * S.rows * 2;
     uint32_t *fblk = faces + (((size_t)bzi * g.nby + byi) * g.nbx + bxi) * k3FaceWords;
 
     if (threadIdx.x < 5) {
@@ -254,10 +257,13 @@ k3_assign(const Geo3 g, const uint8_t *spins, uint32_t *labels, uint32_t *__rest
             sums[threadIdx.x] = 0;
     }
     __syncthreads();
-    if (here)
-        draws_piece3<W, TX>(g, bxi, byi * g.TBY + typ, min(g.py, g.TBY - typ), bzi * g.TBZ + tz, work, D, pairs,
-                            rng_state, rng_sel, rng_iter, thr);
-    __syncwarp();
+    if (exists)
+        draws_piece3<W, TX>(g, bxi, byi * g.TBY + typ, min(g.py, g.TBY - typ), bzi * g.TBZ + tz, work, D, warp / np,
+                            share, pairs, rng_state, rng_sel, rng_iter, thr);
+    if (share == 1)
+        __syncwarp();
+    else
+        __syncthreads();
     after_previous();
 
     // ---- bonds, lane r of a group: row r = kk * PY + j of the piece
@@ -704,6 +710,21 @@ int check_fault3(swb_lattice3 *h)
 
 bool early_launch3(const swb_lattice3 *h) { return h->n_blocks < kEarlyBlocks; }
 
+// Warps that take a piece's draws between them.  A piece of 8-column tiles with W 32 has up to 64 passes, one
+// after the other a large part of a small lattice's sweep: with blocks for at most one SM each, the warps
+// that a CTA may have beyond its pieces help (tile 8 x 1 x 5 with W 32 on 42 x 36 x 2 50 -> 27 us a sweep,
+// 8 x 4 x 4 on 64^3 48 -> 44, the default on 64^3 40 -> 39).  Beyond that the blocks share the SMs: with 256 blocks of
+// 128^3 8 x 8 x 8 tiles 69 -> 91 us, 16 x 4 x 4 on 256^3 182 -> 224.
+constexpr uint32_t k3ShareBlocks = 148;
+template <int W>
+uint32_t draw_share3(const Geo3 &g)
+{
+    if (g.nbx * g.nby * g.nbz > k3ShareBlocks)
+        return 1;
+    const uint32_t passes = (g.py * (32 / g.TX) * W + 31) / 32;
+    return std::max(1u, std::min(passes, k3MaxThreads / 32 / pieces3(g)));
+}
+
 template <int W, int TX>
 int launch_assign3(swb_lattice3 *h, uint32_t thr, uint8_t *dump_bonds, const MeasureArgs &meas)
 {
@@ -711,7 +732,7 @@ int launch_assign3(swb_lattice3 *h, uint32_t thr, uint8_t *dump_bonds, const Mea
     const bool two = g.py * g.TY * g.TZ > 32;
     auto k = two ? (meas.obs ? k3_assign<W, TX, 2, true> : k3_assign<W, TX, 2, false>)
                  : (meas.obs ? k3_assign<W, TX, 1, true> : k3_assign<W, TX, 1, false>);
-    return launch_next(early_launch3(h), k, dim3(g.nbx, g.nby, g.nbz), pieces3(g) * 32, h->smem_assign, h->stream, g,
+    return launch_next(early_launch3(h), k, dim3(g.nbx, g.nby, g.nbz), pieces3(g) * draw_share3<W>(g) * 32, h->smem_assign, h->stream, g,
                        h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, thr, h->faces, dump_bonds, meas);
 }
 
