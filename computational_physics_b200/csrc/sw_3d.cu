@@ -710,19 +710,16 @@ int check_fault3(swb_lattice3 *h)
 
 bool early_launch3(const swb_lattice3 *h) { return h->n_blocks < kEarlyBlocks; }
 
-// Warps that take a piece's draws between them.  A piece of 8-column tiles with W 32 has up to 64 passes, one
-// after the other a large part of a small lattice's sweep: with blocks for at most one SM each, the warps
-// that a CTA may have beyond its pieces help (tile 8 x 1 x 5 with W 32 on 42 x 36 x 2 50 -> 27 us a sweep,
-// 8 x 4 x 4 on 64^3 48 -> 44, the default on 64^3 40 -> 39).  Beyond that the blocks share the SMs: with 256 blocks of
-// 128^3 8 x 8 x 8 tiles 69 -> 91 us, 16 x 4 x 4 on 256^3 182 -> 224.
-constexpr uint32_t k3ShareBlocks = 148;
+// Warps that take a piece's draws between them: where blocks are for at most one SM each, the warps that a CTA
+// may have beyond its pieces help (90 x 76 x 54 with the default tile 57.6 -> 53.4 us a sweep, 8 x 8 x 8 with W 32 on 64^3
+// 60 -> 52).  Beyond that the blocks share the SMs: with 256 blocks of 128^3 8 x 8 x 8 tiles 69 -> 91 us, 16 x 4 x 4 on
+// 256^3 182 -> 224.
 template <int W>
 uint32_t draw_share3(const Geo3 &g)
 {
     if (g.nbx * g.nby * g.nbz > k3ShareBlocks)
         return 1;
-    const uint32_t passes = (g.py * (32 / g.TX) * W + 31) / 32;
-    return std::max(1u, std::min(passes, k3MaxThreads / 32 / pieces3(g)));
+    return std::max(1u, std::min(passes3(g, W), k3MaxThreads / 32 / pieces3(g)));
 }
 
 template <int W, int TX>
@@ -822,7 +819,8 @@ int swb3_create(swb_lattice3 **out, uint32_t L0, uint32_t L1, uint32_t L2, uint3
                     tile_x, tile_y, tile_z);
     if (!(lcg_width == 8 || lcg_width == 16 || lcg_width == 32))
         return fail(SWB_ERR_ARGUMENT, "unsupported lcg32 width %u (8, 16 or 32)", lcg_width);
-    const Geo3 g = make_geo3(L0, L1, L2, tile_x, tile_y, tile_z);
+    Geo3 g = make_geo3(L0, L1, L2, tile_x, tile_y, tile_z);
+    spread3(g, lcg_width);
     if (g.nby > 65535 || g.nbz > 65535)
         return fail(SWB_ERR_ARGUMENT, "lattice of %u x %u x %u sites needs too many block rows or layers", L0, L1, L2);
     swb_lattice3 *h = new swb_lattice3();

@@ -16,6 +16,7 @@ constexpr uint32_t k3MergeThreads = 256;
 constexpr uint32_t k3FlipThreads = 512;   // four quads of a 32 x 16 x 16 block per thread
 constexpr uint32_t k3Window = 256;        // listed unions of a piece worked off at a time
 constexpr uint32_t k3Links = 256;         // linked labels a piece remembers
+constexpr uint32_t k3ShareBlocks = 148;   // up to a block per SM: spread3, draw_share3
 
 struct Geo3 {
     uint32_t L0, L1, L2;        // extent
@@ -26,6 +27,17 @@ struct Geo3 {
     uint32_t nbx, nby, nbz;     // blocks per direction
     uint32_t py, pcy;           // tile rows per piece; pieces per tile layer
 };
+
+// What follows from the tiles per block.
+inline void fit3(Geo3 &g)
+{
+    g.BX = g.TBX * g.TX; g.BY = g.TBY * g.TY; g.BZ = g.TBZ * g.TZ;
+    g.nbx = (g.L0 + g.BX - 1) / g.BX;
+    g.nby = (g.L1 + g.BY - 1) / g.BY;
+    g.nbz = (g.L2 + g.BZ - 1) / g.BZ;
+    g.py = std::min(std::max(1u, 32 / (g.TY * g.TZ)), g.TBY);
+    g.pcy = (g.TBY + g.py - 1) / g.py;
+}
 
 // Blocks of up to 32 x 16 x 16 sites, whole tiles.  Larger blocks have fewer face sites (15.6 % of the
 // sites against 21.9 % with 32 x 8 x 16), which the merge pays for.
@@ -39,13 +51,26 @@ inline Geo3 make_geo3(uint32_t L0, uint32_t L1, uint32_t L2, uint32_t TX, uint32
     g.TBX = std::min(32 / TX, g.n0);
     g.TBY = std::min(k3Rows / TY, g.n1);
     g.TBZ = std::min(k3Layers / TZ, g.n2);
-    g.BX = g.TBX * TX; g.BY = g.TBY * TY; g.BZ = g.TBZ * TZ;
-    g.nbx = (L0 + g.BX - 1) / g.BX;
-    g.nby = (L1 + g.BY - 1) / g.BY;
-    g.nbz = (L2 + g.BZ - 1) / g.BZ;
-    g.py = std::min(std::max(1u, 32 / (TY * TZ)), g.TBY);
-    g.pcy = (g.TBY + g.py - 1) / g.py;
+    fit3(g);
     return g;
+}
+
+// Passes of draws of a piece: its tiles' lanes, a warp at a time.
+__host__ __device__ inline uint32_t passes3(const Geo3 &g, uint32_t W) { return (g.py * (32 / g.TX) * W + 31) / 32; }
+
+// Smaller blocks for a small lattice whose blocks leave half of the SMs idle and would draw in more passes than
+// a CTA has warps: tile 8 x 1 x 3 with W 32 on 38 x 12 x 60 59 -> 27 us a sweep (8 blocks of 400 passes become 64),
+// 8 x 1 x 1 with W 32 on 64^3 70 -> 41, 16 x 2 x 1 on 2 x 16 x 18 30 -> 18.  The default tile's blocks have 16 passes and stay.
+inline void spread3(Geo3 &g, uint32_t W)
+{
+    while (passes3(g, W) * g.pcy * g.TBZ > k3MaxThreads / 32 && 2 * g.nbx * g.nby * g.nbz <= k3ShareBlocks &&
+           g.TBY * g.TBZ > 1) {
+        if (g.TBZ > 1 && (g.BZ >= g.BY || g.TBY == 1))
+            g.TBZ = (g.TBZ + 1) / 2;
+        else
+            g.TBY = (g.TBY + 1) / 2;
+        fit3(g);
+    }
 }
 
 // Face bitmaps of a block: a bit per row (zl * k3Rows + yl) for +x, a word per layer for +y, a word per
@@ -83,8 +108,7 @@ template <int W>
 __host__ __device__ inline Assign3Smem assign3_smem(const Geo3 &g)
 {
     Assign3Smem s{};
-    const uint32_t np = pieces3(g), passes = (g.py * (32 / g.TX) * W + 31) / 32;
-    const uint32_t nd = passes * draws3<W>(g.TX, g.TY, g.TZ).total;
+    const uint32_t np = pieces3(g), nd = passes3(g, W) * draws3<W>(g.TX, g.TY, g.TZ).total;
     s.rows = g.py * g.TY * g.TZ;
     s.wcap = nd > 2 * s.rows ? nd : 2 * s.rows;
     s.wcap = s.wcap > k3Window / 2 ? s.wcap : k3Window / 2;

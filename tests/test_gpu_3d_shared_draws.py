@@ -1,6 +1,7 @@
-"""Small 3D lattices, where several warps take a piece's draws between them (csrc/sw_3d.cu, draw_share3): shares
-of 2 to 16 that do and do not divide the passes, empty passes and pieces, whole and cut tiles, two row groups,
-and the first lattice with more blocks than that.  Bit for bit against the 3D restatement."""
+"""Small 3D lattices, whose blocks are made smaller where they would draw in more passes than a CTA has warps
+(csrc/sw_3d.cuh, spread3) and whose warps take a piece's draws between them (csrc/sw_3d.cu, draw_share3): shares
+that do and do not divide the passes, empty passes and pieces, whole and cut tiles, two row groups, and
+lattices with more blocks than either rule asks for.  Bit for bit against the 3D restatement."""
 import numpy as np
 import pytest
 
@@ -18,8 +19,12 @@ pytestmark = pytest.mark.gpu
     (34, 20, 16, (16, 8, 8), 32),    # 64 rows a piece
     (16, 16, 1, (16, 4, 1), 8),
     (64, 8, 6, (32, 2, 6), 16),
-    (32, 32, 32 * 74, (16, 4, 4), 16),   # 148 x 2 blocks: not shared
-    (32, 32, 32 * 37, (16, 4, 4), 16),   # 148 blocks: shared
+    (38, 12, 60, (8, 1, 3), 32),     # 8 blocks become 64
+    (2, 48, 36, (16, 4, 1), 32),
+    (128, 96, 64, (32, 1, 1), 8),    # 96 blocks of 16 one-row pieces
+    (160, 80, 64, (8, 1, 1), 32),    # 64 passes a piece
+    (32, 32, 16 * 148, (16, 4, 4), 16),  # 296 blocks: not shared
+    (32, 32, 16 * 74, (16, 4, 4), 16),   # 148 blocks: shared
 ])
 def test_shared_draws_bit_exact(gpu, oracle, L0, L1, L2, tile, W):
     spins = np.random.default_rng(L0 + L1 + L2).integers(0, 2, (L2, L1, L0), dtype=np.uint8)
