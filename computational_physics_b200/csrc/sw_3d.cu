@@ -28,7 +28,7 @@
 // every site's label is two lookups away.  A site-by-site form (one union-find node and up to three
 // unions per site) took 12 (default tile on whole blocks) to 31 (any other) warp instructions per
 // site; this one 4.1.  256^3 sweep 397 -> 175 us (assign 278 -> 112, merge 71 -> 32, resolve 37 -> 17), 90 x 76 x
-// 54 169 -> 56 us.
+// 54 169 -> 53 us.
 
 #include <cuda_runtime.h>
 

@@ -69,7 +69,6 @@ struct BatchCounters {
     unsigned int measure_next;    // next entry of the measure list (device work counter)
     unsigned int measure_chunks;  // entries of this round's measure list
     unsigned int n_active;        // lattices in the work lists
-    unsigned int total_chunks;    // measure chunks of all active lattices (the list's capacity)
 };
 
 __device__ __forceinline__ uint32_t next_item(unsigned int *queue, uint32_t *slot)
@@ -566,7 +565,6 @@ int rebuild_lists(swb_batch *b)
     b->grid_round_measure = std::max(1, std::min<int>(b->grid_measure, (int)cp[n]));
     BatchCounters c{};
     c.n_active = n;
-    c.total_chunks = cp[n];
     if (n) {
         SWB_CUDA(cudaMemcpyAsync(b->d_items, items.data(), sizeof(uint2) * items.size(), cudaMemcpyHostToDevice,
                                  b->stream));

@@ -85,7 +85,7 @@ int launch_next(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t 
 // ------------------------------------------------------------------------------------------
 // geometry
 
-// Lattices of at least this many blocks launch their kernels the ordinary way: they fill the GPU for
+// Lattices of at least this many (full-width) blocks launch their kernels the ordinary way: they fill the GPU for
 // longer than a launch takes, and CTAs that wait early hold slots that the running kernel's last
 // waves and other streams' kernels could use (16384^2 sweep 1.44 -> 1.54 ms early; 2048^2 46.3 ->
 // 40.3 us).

@@ -241,7 +241,7 @@ struct swb_lattice {
     uint32_t smem_flip = 0;
     Whole whole{};                 // plain sweeps run as one kernel (whole.ctas != 0)
     bool spins_attached = false;   // spins point at a caller-owned device buffer (swb_attach_spins)
-    bool fused_measure = false;    // the assign phase can measure the spins it starts from
+    bool fused_measure = false;    // samples are taken by the next sweep; false (blocks under 32 columns): by k_measure
     bool measure_pending = false;  // a sample of the current spins is still to be taken
 };
 
@@ -299,8 +299,7 @@ int launch_assign_w(swb_lattice *h, float p_add, const AssignDump &dump, const M
     return launch_assign_k<W, 32, 0>(h, p_add, dump, meas);
 }
 
-// measure: the assign phase also measures the spins it starts from (only where the block
-// labelling uses bond words: fused_measure).
+// measure: the assign phase also measures the spins it starts from (fused_measure).
 int launch_assign(swb_lattice *h, float p_add, const AssignDump &dump = AssignDump{}, bool measure = false)
 {
     const MeasureArgs meas = measure ? MeasureArgs{h->obs, h->series, h->series_cap} : MeasureArgs{};
@@ -523,7 +522,7 @@ int swb_create(swb_lattice **out, uint32_t L0, uint32_t L1, uint32_t tile_x, uin
     SWB_TRY(cudaMemsetAsync(h->spins, 0, h->n + 16, h->stream));
     SWB_TRY(cudaMemsetAsync(h->obs, 0, sizeof(Obs), h->stream));
     h->smem_flip = flip_smem_bytes(h->g);
-    h->fused_measure = (h->g.BX & 31u) == 0 && (h->g.BX & (h->g.BX - 1)) == 0;  // the bond-word labelling
+    h->fused_measure = (h->g.BX & 31u) == 0 && (h->g.BX & (h->g.BX - 1)) == 0;
     h->measure_grid = (int)std::min<size_t>((h->n + 255) / 256, (size_t)sms * 8);
     if (h->measure_grid < 1) h->measure_grid = 1;
     switch (h->W) {

@@ -160,7 +160,8 @@ int swb_launches_per_sweep(swb_lattice *h, uint32_t *launches);
 
 /* n_sweeps sweeps like swb_sweep (no measurement), timed with CUDA events on the handle's
  * stream.  ms[0] = total elapsed; when per_kernel != 0 events bracket every phase and
- * ms[1..3] = summed durations of the assign, merge and resolve + flip kernels.  Synchronous. */
+ * ms[1..3] = summed durations of the assign, merge and resolve + flip kernels; a lattice that
+ * swb_sweep sweeps in one kernel runs its phase kernels then, with identical results.  Synchronous. */
 int swb_sweep_timed(swb_lattice *h, float temperature, uint32_t n_sweeps, int per_kernel, float *ms);
 
 /* Page-locked host memory for fast host<->device copies (cudaHostAlloc / cudaFreeHost). */
