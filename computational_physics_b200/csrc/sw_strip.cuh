@@ -499,21 +499,16 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
     }
 
     // Labels: a block root stores its global site index (the merge links these), every other site
-    // kLocalFlag | the block-local index of its root.  Four sites per lane and row: one 16-byte load of
-    // parents, four lookups, one 16-byte store.  kAny: blocks of one or two strips put four or two rows in a
-    // warp, and rows that are only 8-byte aligned (L0 = 2 mod 4; x0 is a multiple of 8) take two stores,
-    // the second only where the last four columns all lie on the lattice (parent holds own indices behind
-    // it).  With a site per lane and row there instead, 514^2 with 8 x 8 tiles took 43.5 us a sweep, now 33.2.
-    auto store_labels = [&](auto any) {
-        constexpr bool kAny = decltype(any)::value != 0;
-        const uint32_t per = kAny && nstrips <= 2 ? 8 * nstrips : 32;  // lanes of a row
-        const uint32_t x4 = kAny ? lane % per * 4 : lane * 4, y = kAny ? warp * (32 / per) + lane / per : warp;
-        const uint32_t rstep = (blockDim.x >> 5) * (32 / per);
-        const bool whole_quads = !kAny || (g.L0 & 3u) == 0;
+    // kLocalFlag | the block-local index of its root.  (The test is on BX: one on nstrips changes the registers of
+    // whole instances, 960 x 2336 with 16 x 4 tiles 32 -> 40 us a sweep.)
+    if ((g.L0 & 3u) == 0 && g.BX > 32) {
+        // four sites per lane and row: one 16-byte load of parents, four lookups, one 16-byte store
+        // (rows and x0 are 16-byte aligned)
+        const uint32_t x4 = lane * 4, rstep = blockDim.x >> 5;
         if (x4 < bxv) {
-            uint32_t l = y * kBlockPitch + x4, gb = (y0 + y) * g.L0 + x0 + x4;
+            uint32_t l = warp * kBlockPitch + x4, gb = (y0 + warp) * g.L0 + x0 + x4;
 #pragma unroll 2
-            for (uint32_t yl = y; yl < byv; yl += rstep, l += rstep * kBlockPitch, gb += rstep * g.L0) {
+            for (uint32_t yl = warp; yl < byv; yl += rstep, l += rstep * kBlockPitch, gb += rstep * g.L0) {
                 const uint4 pp = *reinterpret_cast<const uint4 *>(parent + l);
                 uint32_t r[4] = {parent[pp.x], parent[pp.y], parent[pp.z], parent[pp.w]};
                 while (deep) {  // the four walks advance together
@@ -532,20 +527,31 @@ __device__ __forceinline__ void assign_strips(const Geo &g, const uint32_t bxi, 
                 o.y = r[1] == l + 1 ? gb + 1 : (kLocalFlag | r[1]);
                 o.z = r[2] == l + 2 ? gb + 2 : (kLocalFlag | r[2]);
                 o.w = r[3] == l + 3 ? gb + 3 : (kLocalFlag | r[3]);
-                if (whole_quads) {
-                    *reinterpret_cast<uint4 *>(labels + gb) = o;
-                } else {
-                    *reinterpret_cast<uint2 *>(labels + gb) = make_uint2(o.x, o.y);
-                    if (x4 + 2 < bxv)
-                        *reinterpret_cast<uint2 *>(labels + gb + 2) = make_uint2(o.z, o.w);
-                }
+                *reinterpret_cast<uint4 *>(labels + gb) = o;
             }
         }
-    };
-    if ((g.L0 & 3u) == 0 && nstrips > 2)
-        store_labels(U32<0>{});
-    else
-        store_labels(U32<1>{});
+    } else if (ncols != 0) {
+        // Rows of L0 = 2 mod 4 are 8-byte aligned (x0 is a multiple of 8), and a block of one strip would leave most
+        // lanes idle above: the warp takes two sites a lane and two rows of its piece at a time.  514^2 with 8 x 8
+        // tiles 43.5 us a sweep with a site a lane and a find for each, now 33; 32 x 262144 at T_c 110 with the loop
+        // above, now 104.
+        const uint32_t x2 = (lane & 15) * 2;
+#pragma unroll 2
+        for (uint32_t yl = r0 + (lane >> 4); x2 < ncols && yl < r0 + rows; yl += 2) {
+            const uint32_t l = yl * kBlockPitch + xs + x2, gb = (y0 + yl) * g.L0 + x0 + xs + x2;
+            const uint2 pp = *reinterpret_cast<const uint2 *>(parent + l);
+            uint32_t ra = parent[pp.x], rb = parent[pp.y];
+            while (deep) {
+                const uint32_t za = parent[ra], zb = parent[rb];
+                if (za == ra && zb == rb)
+                    break;
+                ra = za;
+                rb = zb;
+            }
+            *reinterpret_cast<uint2 *>(labels + gb) =
+                make_uint2(ra == l ? gb : (kLocalFlag | ra), rb == l + 1 ? gb + 1 : (kLocalFlag | rb));
+        }
+    }
     if constexpr (kMeasure) {
         if (threadIdx.x == 0)  // the block's sums (complete since the first barrier)
             obs_add_part(meas.obs, meas.series, meas.cap, (size_t)g.L0 * g.L1, g.nbx * g.nby, sums[0], sums[1], 1);
