@@ -224,7 +224,7 @@ template <int W, int TX, int kGroups, bool kMeasure>
 __global__ void __launch_bounds__(k3MaxThreads, kGroups == 1 ? 2 : 1)
 k3_assign(const Geo3 g, const uint8_t *spins, uint32_t *labels, uint32_t *__restrict__ rng_state,
           uint8_t *__restrict__ rng_sel, uint32_t *__restrict__ rng_iter, const uint32_t thr, uint32_t *faces,
-          uint8_t *dump_bonds, const MeasureArgs meas)
+          uint8_t *dump_bonds, const MeasureArgs meas, const uint32_t share)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const Assign3Smem S = assign3_smem<W>(g);
@@ -241,10 +241,10 @@ k3_assign(const Geo3 g, const uint8_t *spins, uint32_t *labels, uint32_t *__rest
     const size_t plane = (size_t)g.L0 * g.L1;
     // the piece: rows [yp, yp + nj) of layers [zp, zp + nk) of the block.  `share` warps take its draws
     // between them (draw_share3), the first of them all the rest.
-    const uint32_t np = pieces3(g), share = nwarps / np, piece = share == 1 ? warp : warp % np;
+    const uint32_t np = pieces3(g), turn = share == 1 ? 0 : warp / np, piece = warp - turn * np;
     const uint32_t tz = piece / g.pcy, typ = (piece - tz * g.pcy) * g.py;
     const uint32_t yp = typ * g.TY, zp = tz * g.TZ, PY = g.py * g.TY;
-    const bool exists = yp < byv && zp < bzv, here = exists && warp < np;
+    const bool exists = yp < byv && zp < bzv, here = exists && turn == 0;
     const uint32_t nj = here ? min(PY, byv - yp) : 0, nk = here ? min(g.TZ, bzv - zp) : 0;
     uint32_t *work = reinterpret_cast<uint32_t *>(smem + S.work) + piece * S.wcap;
     uint16_t *links = reinterpret_cast<uint16_t *>(smem + S.links) + piece * k3Links;
@@ -258,7 +258,7 @@ k3_assign(const Geo3 g, const uint8_t *spins, uint32_t *labels, uint32_t *__rest
     }
     __syncthreads();
     if (exists)
-        draws_piece3<W, TX>(g, bxi, byi * g.TBY + typ, min(g.py, g.TBY - typ), bzi * g.TBZ + tz, work, D, warp / np,
+        draws_piece3<W, TX>(g, bxi, byi * g.TBY + typ, min(g.py, g.TBY - typ), bzi * g.TBZ + tz, work, D, turn,
                             share, pairs, rng_state, rng_sel, rng_iter, thr);
     if (share == 1)
         __syncwarp();
@@ -727,10 +727,11 @@ int launch_assign3(swb_lattice3 *h, uint32_t thr, uint8_t *dump_bonds, const Mea
 {
     const Geo3 &g = h->g;
     const bool two = g.py * g.TY * g.TZ > 32;
+    const uint32_t share = draw_share3<W>(g);
     auto k = two ? (meas.obs ? k3_assign<W, TX, 2, true> : k3_assign<W, TX, 2, false>)
                  : (meas.obs ? k3_assign<W, TX, 1, true> : k3_assign<W, TX, 1, false>);
-    return launch_next(early_launch3(h), k, dim3(g.nbx, g.nby, g.nbz), pieces3(g) * draw_share3<W>(g) * 32, h->smem_assign, h->stream, g,
-                       h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, thr, h->faces, dump_bonds, meas);
+    return launch_next(early_launch3(h), k, dim3(g.nbx, g.nby, g.nbz), pieces3(g) * share * 32, h->smem_assign, h->stream, g,
+                       h->spins, h->labels, h->rng_state, h->rng_sel, h->rng_iter, thr, h->faces, dump_bonds, meas, share);
 }
 
 template <int W>
